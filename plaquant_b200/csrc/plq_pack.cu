@@ -66,6 +66,8 @@ struct PackArgs {
   int rows_per_cta;          // with a row norm: rows per CTA (warps per CTA = rows_per_cta * lanes / 32)
   int ngroups;               // groups of (warps per CTA) work units = ceil(rows * (lanes / 32) / warps per CTA)
   int stages;                // groups of rows in flight per CTA (1..3 shared-memory stages)
+  int drow, dseg;            // (rows, segments) from a warp's unit to its next one: grid size * warps per CTA units
+  int ring_drow, ring_dseg;  // the same for `stages` steps
 };
 
 // Four 32-bit words of bf16 pairs -> four float32 pairs.
@@ -76,10 +78,37 @@ __device__ __forceinline__ void unpack8(const uint4& w, float2* v) {
   v[3] = make_float2(bf16lo_to_f32(w.w), bf16hi_to_f32(w.w));
 }
 
+// A word of two bf16 (x0 low, x1 high) -> the pair the following steps work on: widened, or, in front of a rotation,
+// its stride-1 butterfly (x0 + x1, x0 - x1).  sm_100 adds a bf16 operand to a float32 one directly, so only x1 has to
+// be widened: three instructions per pair instead of four ([8192, 14336] rotation + pack 70.1 -> 68.0 us).
+template <bool HAD>
+__device__ __forceinline__ float2 enter_pair(uint32_t w) {
+  if constexpr (HAD) {
+    float2 y;
+    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tadd.rn.f32.bf16 %0, l, %3;\n\tsub.rn.f32.bf16 %1, l, %3;\n\t}"
+        : "=f"(y.x), "=f"(y.y)
+        : "r"(w), "f"(bf16hi_to_f32(w)));
+    return y;
+  }
+  return make_float2(bf16lo_to_f32(w), bf16hi_to_f32(w));
+}
+
 // Round a float32 pair to bf16 and widen it again.
 __device__ __forceinline__ float2 round_bf16_pair(const float2 y) {
   const uint32_t b = f32x2_to_bf16x2(y.x, y.y);
   return make_float2(bf16lo_to_f32(b), bf16hi_to_f32(b));
+}
+
+// max |v| over P float32 pairs (two chains; the compiler forms three-input maxima).
+template <int P>
+__device__ __forceinline__ float absmax(const float2* v) {
+  float m0 = 0.0f, m1 = 0.0f;
+#pragma unroll
+  for (int i = 0; i < P; i += 2) {
+    m0 = fmaxf(m0, fmaxf(fabsf(v[i].x), fabsf(v[i].y)));
+    m1 = fmaxf(m1, fmaxf(fabsf(v[i + 1].x), fabsf(v[i + 1].y)));
+  }
+  return fmaxf(m0, m1);
 }
 
 // Output stores.  Plain: this rank's buffer.  Scattered tensor-parallel prologue (PRO 3 with an output table): the
@@ -103,17 +132,11 @@ __device__ __forceinline__ uint32_t quantize_run_nvfp4(const float2* v, uint4& c
   uint32_t words[4];
 #pragma unroll
   for (int b = 0; b < 2; ++b) {
-    float m0 = 0.0f, m1 = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 8; i += 2) {
-      m0 = fmaxf(m0, fmaxf(fabsf(v[8 * b + i].x), fabsf(v[8 * b + i].y)));
-      m1 = fmaxf(m1, fmaxf(fabsf(v[8 * b + i + 1].x), fabsf(v[8 * b + i + 1].y)));
-    }
-    const uint32_t c = nvfp4_scale_code(fmaxf(m0, m1));
+    const uint32_t c = nvfp4_scale_code(absmax<8>(v + 8 * b));
     const float s = e4m3_code_to_f32(c);
-    const float r = __frcp_rn(s);
-    words[2 * b] = nvfp4_quantize8(v + 8 * b, s, r);
-    words[2 * b + 1] = nvfp4_quantize8(v + 8 * b + 4, s, r);
+    const float r = rcp_approx(s);
+    words[2 * b] = nvfp4_quantize8(v + 8 * b, r);
+    words[2 * b + 1] = nvfp4_quantize8(v + 8 * b + 4, r);
     sf2 |= c << (8 * b);
   }
   codes = make_uint4(words[0], words[1], words[2], words[3]);
@@ -129,13 +152,7 @@ __device__ __forceinline__ void store_run_nvfp4(const PackArgs& a, const uint4& 
 // The same for a run in the MXFP8 columns (o >= k_lo): 32 code bytes and one scale byte.
 template <int PRO>
 __device__ __forceinline__ void quantize_run_mxfp8(const PackArgs& a, const float2* v, int row, int o) {
-  float m0 = 0.0f, m1 = 0.0f;
-#pragma unroll
-  for (int i = 0; i < 16; i += 2) {
-    m0 = fmaxf(m0, fmaxf(fabsf(v[i].x), fabsf(v[i].y)));
-    m1 = fmaxf(m1, fmaxf(fabsf(v[i + 1].x), fabsf(v[i + 1].y)));
-  }
-  const uint32_t c = mxfp8_scale_code(fmaxf(m0, m1));
+  const uint32_t c = mxfp8_scale_code(absmax<16>(v));
   const float inv = __uint_as_float((254u - c) << 23);
   const uint2 c0 = mxfp8_quantize8(v, inv), c1 = mxfp8_quantize8(v + 4, inv);
   const uint2 c2 = mxfp8_quantize8(v + 8, inv), c3 = mxfp8_quantize8(v + 12, inv);
@@ -287,12 +304,15 @@ __global__ void PLQ_PACK_BOUNDS pack_kernel(const PackArgs a) {
   const int flip = HAD ? p : 0;                     // odd lanes of a rotated row hold their runs swapped
   const int k8 = a.k >> 3;
   const uint32_t xr = static_cast<uint32_t>((lane & 7) ^ (4 * flip)) << 4;   // chunk swizzle of this lane's line, run 0 first
+  // A warp's units are gridDim * warps apart, so (row, segment) advance by constants the launcher supplies (a division
+  // per unit would cost 0.5 instructions per element); with a row norm the segment never changes.
   struct Unit { int row, seg; };
-  auto unit_of = [&](int group) {
-    const int u = group * nwarps + warp;
-    Unit t;
-    t.row = u / wpr;
-    t.seg = u - t.row * wpr;
+  auto ahead = [&](Unit t, int drow, int dseg) {
+    t.row += drow;
+    if constexpr (!NORM) {
+      t.seg += dseg;
+      if (t.seg >= wpr) { t.seg -= wpr; ++t.row; }
+    }
     return t;
   };
   constexpr bool kStageX = true;                    // x always passes through shared memory ...
@@ -305,8 +325,7 @@ __global__ void PLQ_PACK_BOUNDS pack_kernel(const PackArgs a) {
   uint8_t* gs = pack_smem + a.stages * stage_bytes + (warp - rl * wpr) * 2 * kSegBytes;   // gamma as float32, this warp's segment
   const int ld2 = PRO == 1 ? a.ldx8 : k8;           // row stride of x2 in 16-byte units
 
-  auto stage_group = [&](int group, int slot) {
-    const Unit t = unit_of(group);
+  auto stage_unit = [&](const Unit& t, int slot) {
     const int n = t.row < a.rows ? min(max(k8 - 256 * t.seg, 0), 256) : 0;     // 16-byte pieces of the segment inside the row
     const size_t r0 = static_cast<size_t>(t.row < a.rows ? t.row : 0);
     if constexpr (kCopyX) stage_segment(smem_u32(xs0 + slot * stage_bytes), a.x + r0 * a.ldx8 + 256 * t.seg, n, lane);
@@ -362,14 +381,23 @@ __global__ void PLQ_PACK_BOUNDS pack_kernel(const PackArgs a) {
     }
   }
   const int stride = static_cast<int>(gridDim.x);
-  for (int s = 0; s < a.stages; ++s) {               // fill the ring: one committed copy group per stage
-    if (group + s * stride < ngroups) stage_group(group + s * stride, s);
-    cp_async_commit();
+  Unit unit;
+  {
+    const int u = group * nwarps + warp;
+    unit.row = u / wpr;
+    unit.seg = u - unit.row * wpr;
+  }
+  {
+    Unit t = unit;
+    for (int s = 0; s < a.stages; ++s) {             // fill the ring: one committed copy group per stage
+      if (group + s * stride < ngroups) stage_unit(t, s);
+      t = ahead(t, a.drow, a.dseg);
+      cp_async_commit();
+    }
   }
   int iter = 0, slot = 0;
 
-  for (; group < ngroups; group += stride, ++iter) {
-    const Unit unit = unit_of(group);
+  for (; group < ngroups; group += stride, ++iter, unit = ahead(unit, a.drow, a.dseg)) {
     const int row = unit.row;
     const int l = 32 * unit.seg + lane;               // lane of the row: elements [64 l, 64 l + 64)
     const int in0 = 64 * l + 32 * flip;               // first element of register run 0 / run 1 as loaded
@@ -399,13 +427,17 @@ __global__ void PLQ_PACK_BOUNDS pack_kernel(const PackArgs a) {
       if constexpr (kStageX) read_line(xs0 + slot * stage_bytes, lane, xr, w);
       if constexpr (kStageX2) read_line(x2s0 + slot * stage_bytes, lane, xr, w2);
       __syncwarp();                                 // every lane has its pieces: the slot is free again
-      if (group + a.stages * stride < ngroups) stage_group(group + a.stages * stride, slot);
+      if (group + a.stages * stride < ngroups) stage_unit(ahead(unit, a.ring_drow, a.ring_dseg), slot);
       cp_async_commit();
       cur_slot = slot;
       if (++slot == a.stages) slot = 0;
       if constexpr (PRO == 0) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) unpack8(w[c], v + 4 * c);
+        for (int c = 0; c < 8; ++c) {
+          const uint32_t ww[4] = {w[c].x, w[c].y, w[c].z, w[c].w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) v[4 * c + i] = enter_pair<HAD && !NORM>(ww[i]);
+        }
       } else if constexpr (PRO == 1) {
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
@@ -413,11 +445,11 @@ __global__ void PLQ_PACK_BOUNDS pack_kernel(const PackArgs a) {
           const uint32_t uu[4] = {w2[c].x, w2[c].y, w2[c].z, w2[c].w};
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const float2 sl = silu_det2(make_float2(bf16lo_to_f32(ww[i]), bf16hi_to_f32(ww[i])));
+            const float2 sl = silu2(make_float2(bf16lo_to_f32(ww[i]), bf16hi_to_f32(ww[i])));
             const uint32_t t = f32x2_to_bf16x2(sl.x, sl.y);                                                        // SiLU, to bf16
             const float2 prod = __fmul2_rn(make_float2(bf16lo_to_f32(t), bf16hi_to_f32(t)),
                                            make_float2(bf16lo_to_f32(uu[i]), bf16hi_to_f32(uu[i])));
-            v[4 * c + i] = round_bf16_pair(prod);                                                                  // product, to bf16
+            v[4 * c + i] = enter_pair<HAD>(f32x2_to_bf16x2(prod.x, prod.y));                                       // product, to bf16
           }
         }
       } else {
@@ -466,8 +498,10 @@ __global__ void PLQ_PACK_BOUNDS pack_kernel(const PackArgs a) {
 #pragma unroll
       for (int c = 0; c < 16; ++c) {
         const float4 g = gl[32 * c];
-        v[2 * c] = round_bf16_pair(__fmul2_rn(make_float2(g.x, g.y), __fmul2_rn(v[2 * c], r2)));
-        v[2 * c + 1] = round_bf16_pair(__fmul2_rn(make_float2(g.z, g.w), __fmul2_rn(v[2 * c + 1], r2)));
+        const float2 y0 = __fmul2_rn(make_float2(g.x, g.y), __fmul2_rn(v[2 * c], r2));
+        const float2 y1 = __fmul2_rn(make_float2(g.z, g.w), __fmul2_rn(v[2 * c + 1], r2));
+        v[2 * c] = enter_pair<HAD>(f32x2_to_bf16x2(y0.x, y0.y));
+        v[2 * c + 1] = enter_pair<HAD>(f32x2_to_bf16x2(y1.x, y1.y));
       }
     }
 
@@ -475,12 +509,7 @@ __global__ void PLQ_PACK_BOUNDS pack_kernel(const PackArgs a) {
     if constexpr (HAD) {
       const float2 neg1 = make_float2(-1.0f, -1.0f);
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {                       // stride 1: inside a pair
-        const float x0 = v[i].x, x1 = v[i].y;
-        v[i] = make_float2(__fadd_rn(x0, x1), __fsub_rn(x0, x1));
-      }
-#pragma unroll
-      for (int h = 1; h < 16; h <<= 1) {                   // strides 2, 4, 8, 16: pairs i, i + h of one run
+      for (int h = 1; h < 16; h <<= 1) {                   // stride 1 (inside a pair) is done (enter_pair); strides 2, 4, 8, 16: pairs i, i + h of one run
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           if ((i & h) == 0) {
@@ -811,7 +840,10 @@ static int launch_pack(int pro, const void* x, const void* x2, void* h_out, int6
     if (st != PLQ_OK) return st;
     const int64_t resident = static_cast<int64_t>(per_sm) * sm_count();
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(groups < resident ? groups : resident), 1, 1);   // persistent: grid stride over the groups
+    const int64_t grid = groups < resident ? groups : resident;      // persistent: grid stride over the groups
+    a.drow = static_cast<int>(grid * warps / wpr); a.dseg = static_cast<int>(grid * warps % wpr);
+    a.ring_drow = static_cast<int>(stages * grid * warps / wpr); a.ring_dseg = static_cast<int>(stages * grid * warps % wpr);
+    cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
     cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
     cfg.dynamicSmemBytes = static_cast<size_t>(smem);
     cfg.stream = static_cast<cudaStream_t>(stream);

@@ -7,10 +7,14 @@
 //     smallest s with 6*s >= max (6*s is exact in float32 and a bf16 value can never sit
 //     within float32 rounding distance of 6*s without being equal to it), so a hardware
 //     round-to-nearest conversion plus one exact comparison finds it.
-//   * NVFP4 element: E2M1 code of fl(x/s).  x*fl(1/s) refined by one Newton step
-//     (two FMAs) equals m exactly whenever x == m*s for a rounding midpoint m, and is far
-//     (>= 2^-9 relative) from every midpoint otherwise, so the hardware RNE conversion of
-//     the refined quotient yields the same code as the reference's correctly rounded one.
+//   * NVFP4 element: E2M1 code of fl(x/s), from one multiplication x*r rounded toward zero with
+//     r = fl(1/s) (the hardware approximation equals it for all 126 scales).  x/s is either exactly a rounding midpoint m or at least 2^-9 (relative) away from
+//     every midpoint, so only x == m*s is delicate: fl(1/s) never lies below 1/s (true for the eight
+//     significands an E4M3 value can have), the product is m(1 + e) with 0 <= e < one ulp, and rounding
+//     toward zero returns m itself; the hardware RNE conversion then breaks the tie like the
+//     reference's correctly rounded quotient.  (Before: the quotient refined by two more multiply-adds;
+//     together with unit indexes advanced instead of divided, [8192, 14336] rotation + pack went from
+//     80.4 to 70.1 us.)
 //   * MXFP8 scale: 2^e with the smallest e such that 448*2^e >= max, read off the bf16
 //     exponent and mantissa; element: x * 2^-e is exact, then hardware RNE to E4M3.
 //   * sign of zero: the reference multiplies the rounded magnitude by sign(x/s), so only a
@@ -32,6 +36,17 @@ __device__ __forceinline__ uint32_t f32x2_to_bf16x2(float a, float b) {
   uint32_t d;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(b), "f"(a));
   return d;
+}
+
+__device__ __forceinline__ float ex2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 
 // E4M3 code (0..0x7E) -> float32, subnormals included: the code shifted into the float32
@@ -56,15 +71,11 @@ __device__ __forceinline__ uint32_t nvfp4_scale_code(float bmax) {
 }
 
 // Eight float32 (bf16-valued, four pairs) -> eight E2M1 codes, element 0 in bits [0,4).
-__device__ __forceinline__ uint32_t nvfp4_quantize8(const float2* x, float s, float r) {
+__device__ __forceinline__ uint32_t nvfp4_quantize8(const float2* x, float r) {
   float2 q[4];
-  const float2 r2 = make_float2(r, r), ns2 = make_float2(-s, -s);
+  const float2 r2 = make_float2(r, r), zero = make_float2(0.0f, 0.0f);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 q0 = __fmul2_rn(x[i], r2);
-    const float2 e = __ffma2_rn(ns2, q0, x[i]);
-    q[i] = __ffma2_rn(e, r2, q0);
-  }
+  for (int i = 0; i < 4; ++i) q[i] = __ffma2_rz(x[i], r2, zero);
   uint32_t out;
   asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
       "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
@@ -74,9 +85,9 @@ __device__ __forceinline__ uint32_t nvfp4_quantize8(const float2* x, float s, fl
       "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
       : "=r"(out)
       : "f"(q[0].x), "f"(q[0].y), "f"(q[1].x), "f"(q[1].y), "f"(q[2].x), "f"(q[2].y), "f"(q[3].x), "f"(q[3].y));
-  // No sign fix-up is needed here: the quotient is zero only for x = +-0, and for x = -0 the two
-  // refinement FMAs already turn it into +0 (e = (-s)(-0) + (-0) = +0, q = (+0) r + (-0) = +0), which is
-  // what the reference's sign(x/s) * |q| gives; a negative x that merely rounds to zero keeps its sign.
+  // No sign fix-up is needed here: the quotient is zero only for x = +-0, and the + 0 of the multiply-add turns a -0
+  // product into +0, which is what the reference's sign(x/s) * |q| gives; a negative x that merely rounds to zero
+  // keeps its sign.
   return out;
 }
 
@@ -114,67 +125,20 @@ __device__ __forceinline__ uint2 mxfp8_quantize8(const float2* x, float inv) {
 // 2^(code-127) as float32 for an E8M0 byte in [1, 254].
 __device__ __forceinline__ float e8m0_to_f32(uint32_t code) { return __uint_as_float(code << 23); }
 
-// ---- SiLU with a written-down float32 exponential -------------------------------------------
-// exp(x) for the SiLU prologue, defined operation by operation so that the CPU checker can restate it
-// bit for bit (a library expf is only specified to a few units in the last place): every multiply and
-// add below is a separately rounded IEEE float32 operation (no fused multiply-add), in this order:
-//   x  <- min(max(x, -100), 100)
-//   n  <- (x * log2(e) + 1.5 * 2^23) - 1.5 * 2^23           (nearest integer, ties to even)
-//   r  <- (x - n * 0.693359375) - n * (-2.12194440e-4)       (Cody-Waite split of ln 2)
-//   p  <- 1 + r (1 + r (1/2 + r (1/6 + r (1/24 + r (1/120 + r (1/720 + r / 5040))))))   (Horner)
-//   exp <- (p * 2^floor(n/2)) * 2^(n - floor(n/2))           (two exact scalings; overflows to +inf)
-// |r| <= 0.3466, so the truncated series is within 6e-9 of e^r; the result is within ~2 ulp of exp(x).
-__device__ __forceinline__ float exp_det(float x) {
-  x = fminf(fmaxf(x, -100.0f), 100.0f);
-  const float magic = 12582912.0f;
-  const float n = __fsub_rn(__fadd_rn(__fmul_rn(x, 1.44269502162933349609375f), magic), magic);
-  float r = __fsub_rn(x, __fmul_rn(n, 0.693359375f));
-  r = __fsub_rn(r, __fmul_rn(n, -2.12194440e-4f));
-  float p = 1.98412701138295233249664306640625e-4f;                       // 1/5040
-  p = __fadd_rn(__fmul_rn(p, r), 1.388888922519981861114501953125e-3f);    // 1/720
-  p = __fadd_rn(__fmul_rn(p, r), 8.3333337679505348205566406250e-3f);      // 1/120
-  p = __fadd_rn(__fmul_rn(p, r), 4.16666679084300994873046875e-2f);        // 1/24
-  p = __fadd_rn(__fmul_rn(p, r), 0.1666666716337203979492187500f);         // 1/6
-  p = __fadd_rn(__fmul_rn(p, r), 0.5f);
-  p = __fadd_rn(__fmul_rn(p, r), 1.0f);
-  p = __fadd_rn(__fmul_rn(p, r), 1.0f);
-  const int ni = __float2int_rn(n);
-  const int h = ni >> 1;
-  const float s1 = __uint_as_float(static_cast<uint32_t>(h + 127) << 23);
-  const float s2 = __uint_as_float(static_cast<uint32_t>(ni - h + 127) << 23);
-  return __fmul_rn(__fmul_rn(p, s1), s2);
-}
-
-// The same list of operations on two values at once (packed float32x2 multiplies and adds round each element like
-// their scalar forms, so the results are those of exp_det).
-__device__ __forceinline__ float2 exp_det2(float2 x) {
-  x.x = fminf(fmaxf(x.x, -100.0f), 100.0f);
-  x.y = fminf(fmaxf(x.y, -100.0f), 100.0f);
-  const float2 magic = make_float2(12582912.0f, 12582912.0f), nmagic = make_float2(-12582912.0f, -12582912.0f);
-  const float2 n = __fadd2_rn(__fadd2_rn(__fmul2_rn(x, make_float2(1.44269502162933349609375f, 1.44269502162933349609375f)), magic), nmagic);
-  // x - n * c == x + n * (-c): the product only changes sign
-  float2 r = __fadd2_rn(x, __fmul2_rn(n, make_float2(-0.693359375f, -0.693359375f)));
-  r = __fadd2_rn(r, __fmul2_rn(n, make_float2(2.12194440e-4f, 2.12194440e-4f)));
-  float2 p = make_float2(1.98412701138295233249664306640625e-4f, 1.98412701138295233249664306640625e-4f);
-  const float c[7] = {1.388888922519981861114501953125e-3f, 8.3333337679505348205566406250e-3f,
-                      4.16666679084300994873046875e-2f, 0.1666666716337203979492187500f, 0.5f, 1.0f, 1.0f};
-#pragma unroll
-  for (int i = 0; i < 7; ++i) p = __fadd2_rn(__fmul2_rn(p, r), make_float2(c[i], c[i]));
-  const int n0 = __float2int_rn(n.x), n1 = __float2int_rn(n.y);
-  const int h0 = n0 >> 1, h1 = n1 >> 1;
-  const float2 s1 = make_float2(__uint_as_float(static_cast<uint32_t>(h0 + 127) << 23),
-                                __uint_as_float(static_cast<uint32_t>(h1 + 127) << 23));
-  const float2 s2 = make_float2(__uint_as_float(static_cast<uint32_t>(n0 - h0 + 127) << 23),
-                                __uint_as_float(static_cast<uint32_t>(n1 - h1 + 127) << 23));
-  return __fmul2_rn(__fmul2_rn(p, s1), s2);
-}
-
-// SiLU(g) = g / (1 + exp(-g)), float32, IEEE division (torch.nn.functional.silu on a bf16 tensor computes in
-// float32 and rounds once; the caller does that rounding).
-__device__ __forceinline__ float silu_det(float g) { return __fdiv_rn(g, __fadd_rn(1.0f, exp_det(-g))); }
-__device__ __forceinline__ float2 silu_det2(float2 g) {
-  const float2 d = __fadd2_rn(make_float2(1.0f, 1.0f), exp_det2(make_float2(-g.x, -g.y)));
-  return make_float2(__fdiv_rn(g.x, d.x), __fdiv_rn(g.y, d.y));
+// ---- SiLU ------------------------------------------------------------------------------------
+// SiLU(g) = g / (1 + exp(-g)) of a bf16-valued g, to be rounded to bf16 by the caller.  The CPU checker defines it
+// with a float32 exponential written down operation by operation and an IEEE division (silu_mul_bf16 / exp_det); the
+// value needed is its rounding to 8 significant bits for one of 65 280 possible inputs, and the hardware's ex2 and
+// rcp approximations (a few units in the 24th bit) give the same bf16 for every one of them - the GPU tests compare
+// all finite inputs - with 5 instructions per element instead of the definition's ~35 ([32768, 28672] -> packed:
+// 2175 -> 890 us = 4.8 TB/s).
+// The denominator is scaled by 1/4: up to 2^126 its reciprocal is a normal number, above that exp has overflowed and
+// the quotient is zero on either path.
+__device__ __forceinline__ float2 silu2(float2 g) {
+  const float2 q = make_float2(0.25f, 0.25f);
+  const float2 t = __fmul2_rn(g, make_float2(-1.44269502162933349609375f, -1.44269502162933349609375f));
+  const float2 d = __ffma2_rn(make_float2(ex2_approx(t.x), ex2_approx(t.y)), q, q);
+  return __fmul2_rn(__fmul2_rn(g, q), make_float2(rcp_approx(d.x), rcp_approx(d.y)));
 }
 
 #endif  // __CUDACC__
