@@ -74,7 +74,9 @@ def check_device_status(device=None) -> None:
         _lib.check(v)
 
 
-def alloc_packed(rows: int, k: int, k_hi: int, sf_layout, device) -> PackedMatrix:
+def alloc_packed(rows: int, k: int, k_hi: int, sf_layout, device, zero_padding: bool = True) -> PackedMatrix:
+    """Buffers for a packed [rows, k] matrix.  `zero_padding=False`: the pack kernels are going to fill them (they write
+    the padding scales themselves)."""
     layout = _LAYOUTS[sf_layout]
     k_lo = k - k_hi
     L = _lib.lib()
@@ -85,7 +87,7 @@ def alloc_packed(rows: int, k: int, k_hi: int, sf_layout, device) -> PackedMatri
         # 0 x NaN is NaN: they must be zero.  K_lo / 16 is always a multiple of four; K_hi / 32 need not be.
         lo_sf = torch.empty(L.plq_sf_tiled_bytes(rows, k_lo // 16), **u8)
         hi_bytes = L.plq_sf_tiled_bytes(rows, k_hi // 32)
-        hi_sf = torch.zeros(hi_bytes, **u8) if (k_hi // 32) % 4 else torch.empty(hi_bytes, **u8)
+        hi_sf = torch.zeros(hi_bytes, **u8) if zero_padding and (k_hi // 32) % 4 else torch.empty(hi_bytes, **u8)
     else:
         lo_sf = torch.empty(rows, k_lo // 16, **u8)
         hi_sf = torch.empty(rows, k_hi // 32, **u8)
@@ -105,7 +107,7 @@ def pack(x: torch.Tensor, k_hi: int, hadamard: bool = False, sf_layout="tiled",
     if not x2.is_contiguous():
         x2 = x2.contiguous()
     rows = x2.shape[0]
-    p = out if out is not None else alloc_packed(rows, k, k_hi, sf_layout, x.device)
+    p = out if out is not None else alloc_packed(rows, k, k_hi, sf_layout, x.device, zero_padding=False)
     L = _lib.lib()
     with torch.cuda.device(x.device):
         if gamma is None:
@@ -134,7 +136,7 @@ def silu_mul_pack(gate_up: torch.Tensor, k_hi: int, hadamard: bool = True, sf_la
     if not g2.is_contiguous():
         g2 = g2.contiguous()
     rows = g2.shape[0]
-    p = out if out is not None else alloc_packed(rows, k, k_hi, sf_layout, gate_up.device)
+    p = out if out is not None else alloc_packed(rows, k, k_hi, sf_layout, gate_up.device, zero_padding=False)
     with torch.cuda.device(gate_up.device):
         st = _lib.lib().plq_silu_mul_pack(_ptr(g2), g2.data_ptr() + 2 * k if rows else None, 2 * k, rows, k, k_hi,
                                           int(hadamard), _ptr(p.lo_codes), _ptr(p.lo_sf), _ptr(p.hi_codes),
@@ -155,7 +157,7 @@ def add_rmsnorm_pack(x: torch.Tensor, residual: torch.Tensor, gamma: torch.Tenso
     x2, r2 = x.reshape(-1, k).contiguous(), residual.reshape(-1, k).contiguous()
     rows = x2.shape[0]
     h = torch.empty_like(x2)
-    p = out if out is not None else alloc_packed(rows, k, k_hi, sf_layout, x.device)
+    p = out if out is not None else alloc_packed(rows, k, k_hi, sf_layout, x.device, zero_padding=False)
     if gamma.dtype != torch.bfloat16 or gamma.numel() != k:
         raise TypeError("gamma must be bfloat16 [K]")
     with torch.cuda.device(x.device):
@@ -179,7 +181,7 @@ def allreduce_add_rmsnorm_pack(peer, rows: int, residual: torch.Tensor, gamma: t
     if gamma.dtype != torch.bfloat16 or gamma.numel() != k:
         raise TypeError("gamma must be bfloat16 [K]")
     h = torch.empty_like(r2)
-    p = out if out is not None else alloc_packed(rows, k, k_hi, sf_layout, residual.device)
+    p = out if out is not None else alloc_packed(rows, k, k_hi, sf_layout, residual.device, zero_padding=False)
     with torch.cuda.device(residual.device):
         st = _lib.lib().plq_allreduce_add_rmsnorm_pack(
             _ptr(peer.peer_x[peer.next]), _ptr(peer.peer_flags), _ptr(peer.flags), _ptr(peer.sync), peer.world, peer.rank,
