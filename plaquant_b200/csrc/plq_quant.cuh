@@ -70,6 +70,16 @@ __device__ __forceinline__ uint32_t nvfp4_scale_code(float bmax) {
   return min(c, 0x7Eu);              // saturate at 448, never the NaN code
 }
 
+// Two float32 (bf16-valued) -> two E2M1 codes, the first in bits [0,4); r as in nvfp4_quantize8.
+__device__ __forceinline__ uint32_t nvfp4_quantize2(const float2 x, float r) {
+  const float2 q = __ffma2_rz(x, make_float2(r, r), make_float2(0.0f, 0.0f));
+  uint32_t out;
+  asm("{\n\t.reg .b8 b0;\n\tcvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\tmov.b32 %0, {b0, b0, b0, b0};\n\t}"
+      : "=r"(out)
+      : "f"(q.x), "f"(q.y));
+  return out & 0xFFu;
+}
+
 // Eight float32 (bf16-valued, four pairs) -> eight E2M1 codes, element 0 in bits [0,4).
 __device__ __forceinline__ uint32_t nvfp4_quantize8(const float2* x, float r) {
   float2 q[4];

@@ -9,6 +9,7 @@
 //     out[64 + i] = x2 * cos[64 + i] +   x1  * sin[64 + i]
 // which is `x.float() * cos + rotate_half(x).float() * sin` of the PyTorch formulation, bit for bit.
 #include "plq_common.cuh"
+#include "plq_quant.cuh"
 
 namespace plq {
 
@@ -93,21 +94,133 @@ __global__ void __launch_bounds__(256, 6) rope_kv_append_kernel(const RopeArgs a
   dst[8] = hi;
 }
 
-}  // namespace plq
+// ---- the same with a packed cache ------------------------------------------------------------------------------
+// Rows of the NVFP4 cache: 64 bytes of E2M1 codes, 8 E4M3 scale bytes.  One warp per head row, lane l holding elements
+// (2 l, 2 l + 1) and (64 + 2 l, 65 + 2 l): RoPE and the last butterfly stage stay in the lane, a 16-element block is
+// eight lanes.  Replaces, per decode step and layer, fifteen elementwise, pack and concatenation launches over a few
+// hundred rows each; those were bound by their launches.
+constexpr int kPackedRow = 72;
 
-extern "C" int plq_rope_kv_append(const void* qkv_bf16, int64_t ld, const void* cos_f32, const void* sin_f32,
-                                  int64_t batch, int64_t t, int64_t heads, int64_t kv_heads, int64_t head_dim,
-                                  void* q_out_bf16, void* k_cache_bf16, void* v_cache_bf16, int64_t t_max,
-                                  const int64_t* pos_dev, int64_t pos, int32_t* dev_status, void* stream) {
-  using namespace plq;
+struct HeadRow { float2 a, b; };
+
+__device__ __forceinline__ HeadRow bf16_row(float2 a, float2 b) {
+  const uint32_t w0 = f32x2_to_bf16x2(a.x, a.y), w1 = f32x2_to_bf16x2(b.x, b.y);
+  return {make_float2(bf16lo_to_f32(w0), bf16hi_to_f32(w0)), make_float2(bf16lo_to_f32(w1), bf16hi_to_f32(w1))};
+}
+__device__ __forceinline__ HeadRow rope_row(const HeadRow& x, const float* cos, const float* sin, int lane) {
+  const float2 c1 = *reinterpret_cast<const float2*>(cos + 2 * lane), c2 = *reinterpret_cast<const float2*>(cos + 64 + 2 * lane);
+  const float2 s1 = *reinterpret_cast<const float2*>(sin + 2 * lane), s2 = *reinterpret_cast<const float2*>(sin + 64 + 2 * lane);
+  float2 lo, hi;
+  lo.x = __fadd_rn(__fmul_rn(x.a.x, c1.x), __fmul_rn(-x.b.x, s1.x));
+  lo.y = __fadd_rn(__fmul_rn(x.a.y, c1.y), __fmul_rn(-x.b.y, s1.y));
+  hi.x = __fadd_rn(__fmul_rn(x.b.x, c2.x), __fmul_rn(x.a.x, s2.x));
+  hi.y = __fadd_rn(__fmul_rn(x.b.y, c2.y), __fmul_rn(x.a.y, s2.y));
+  return bf16_row(lo, hi);
+}
+// Block-Hadamard(128), stages of stride 1, 2, .. 64 in this order and one rounding to bf16: bit for bit the rotation
+// of the pack kernels (up to the sign of a zero, which the quantiser drops).
+__device__ __forceinline__ HeadRow hadamard_row(HeadRow x, int lane) {
+  x.a = make_float2(__fadd_rn(x.a.x, x.a.y), __fsub_rn(x.a.x, x.a.y));
+  x.b = make_float2(__fadd_rn(x.b.x, x.b.y), __fsub_rn(x.b.x, x.b.y));
+#pragma unroll
+  for (int h = 1; h < 32; h <<= 1) {
+    const bool up = (lane & h) != 0;               // this lane holds the upper element: partner - own
+    float* e[4] = {&x.a.x, &x.a.y, &x.b.x, &x.b.y};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float o = __shfl_xor_sync(0xFFFFFFFFu, *e[i], h);
+      *e[i] = up ? __fsub_rn(o, *e[i]) : __fadd_rn(*e[i], o);
+    }
+  }
+  const float c = 0.088388347648318441f;           // 1/sqrt(128)
+  return bf16_row(make_float2(__fmul_rn(__fadd_rn(x.a.x, x.b.x), c), __fmul_rn(__fadd_rn(x.a.y, x.b.y), c)),
+                  make_float2(__fmul_rn(__fsub_rn(x.a.x, x.b.x), c), __fmul_rn(__fsub_rn(x.a.y, x.b.y), c)));
+}
+__device__ __forceinline__ void store_nvfp4_row(uint8_t* p, const HeadRow& x, int lane) {
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const float2 v = half ? x.b : x.a;
+    float m = fmaxf(fabsf(v.x), fabsf(v.y));
+    m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, 1));
+    m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, 2));
+    m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, 4));
+    const uint32_t c = nvfp4_scale_code(m);
+    p[32 * half + lane] = static_cast<uint8_t>(nvfp4_quantize2(v, rcp_approx(e4m3_code_to_f32(c))));
+    if ((lane & 7) == 0) p[64 + 4 * half + (lane >> 3)] = static_cast<uint8_t>(c);
+  }
+}
+
+__global__ void __launch_bounds__(256) rope_kv_append_nvfp4_kernel(const RopeArgs a) {
+  const long long idx = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;      // head row
+  if (idx >= a.total) return;
+  const int lane = threadIdx.x & 31;
+  const int all_heads = a.heads + 2 * a.kv_heads;
+  const int head = static_cast<int>(idx % all_heads);
+  const long long row = idx / all_heads;
+  const long long b = row / a.t;
+  const int tt = static_cast<int>(row - b * a.t);
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(a.qkv + row * a.ld8 + static_cast<long long>(head) * 16) + lane;
+  const uint32_t w0 = src[0], w1 = src[32];
+  HeadRow x = {make_float2(bf16lo_to_f32(w0), bf16hi_to_f32(w0)), make_float2(bf16lo_to_f32(w1), bf16hi_to_f32(w1))};
+  const bool is_q = head < a.heads, is_k = !is_q && head < a.heads + a.kv_heads;
+  if (is_q || is_k) x = rope_row(x, a.cos + static_cast<size_t>(tt) * kRopeHeadDim, a.sin + static_cast<size_t>(tt) * kRopeHeadDim, lane);
+  if (is_q) {
+    uint32_t* dst = reinterpret_cast<uint32_t*>(a.q_out + (row * a.heads + head) * 16) + lane;
+    dst[0] = f32x2_to_bf16x2(x.a.x, x.a.y);
+    dst[32] = f32x2_to_bf16x2(x.b.x, x.b.y);
+    return;
+  }
+  const long long p = (a.pos_dev != nullptr ? *a.pos_dev : a.pos) + tt;
+  if (p < 0 || p >= a.t_max) {                       // the cache is full: nothing is stored, the caller is told
+    if (lane == 0 && a.status != nullptr) atomicExch(a.status, PLQ_DEV_RANGE);
+    return;
+  }
+  if (is_k) x = hadamard_row(x, lane);
+  const int kh = head - a.heads - (is_k ? 0 : a.kv_heads);
+  store_nvfp4_row(reinterpret_cast<uint8_t*>(is_k ? a.k_dst : a.v_dst) + ((b * a.t_max + p) * a.kv_heads + kh) * kPackedRow, x, lane);
+}
+
+// Packed rows of keys and values -> their bf16 values, both caches in one launch, straight out of caches with room for
+// t_max positions: eight elements (four code bytes, one scale byte) per thread, 16-byte stores.  A code times its scale
+// has at most 7 significant bits, so the bf16 value is exact (and equal to plq_unpack's).  Bound by the bytes written
+// (256 per 72 read).
+struct UnpackRowsArgs {
+  const uint8_t* src[2];     // [batch, t_max, kv_heads, 72]
+  uint4* dst[2];             // bf16 [batch, t, kv_heads, 128]
+  long long t_heads, cap_heads, total;     // t * kv_heads, t_max * kv_heads, threads per cache = batch * t * kv_heads * 16
+};
+
+__global__ void __launch_bounds__(256) unpack_head_rows_kernel(const UnpackRowsArgs a) {
+  const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (idx >= a.total) return;
+  const long long r = idx >> 4, b = r / a.t_heads;
+  const int j = static_cast<int>(idx & 15);
+  const uint8_t* p = (blockIdx.y == 0 ? a.src[0] : a.src[1]) + (b * a.cap_heads + (r - b * a.t_heads)) * kPackedRow;
+  const uint32_t codes = *reinterpret_cast<const uint32_t*>(p + 4 * j);
+  const float s = e4m3_code_to_f32(p[64 + (j >> 1)]);
+  float f[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t c = (codes >> (4 * i)) & 0xF, mag = c & 7;
+    const float mv = mag < 2 ? 0.5f * mag : __uint_as_float(((mag >> 1) + 126u) << 23 | (mag & 1u) << 22);
+    f[i] = (c & 8) ? -(mv * s) : mv * s;
+  }
+  (blockIdx.y == 0 ? a.dst[0] : a.dst[1])[idx] = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+}
+
+
+static int launch_rope(bool packed, const void* qkv_bf16, int64_t ld, const void* cos_f32, const void* sin_f32,
+                       int64_t batch, int64_t t, int64_t heads, int64_t kv_heads, int64_t head_dim,
+                       void* q_out_bf16, void* k_cache, void* v_cache, int64_t t_max,
+                       const int64_t* pos_dev, int64_t pos, int32_t* dev_status, void* stream) {
   if (head_dim != kRopeHeadDim) return PLQ_ERR_SHAPE;
   if (batch < 1 || t < 1 || heads < 1 || kv_heads < 1 || t_max < 1) return PLQ_ERR_SHAPE;
   if (ld < (heads + 2 * kv_heads) * kRopeHeadDim || ld % 8 != 0) return PLQ_ERR_SHAPE;
   if (pos_dev == nullptr && (pos < 0 || pos + t > t_max)) return PLQ_ERR_SHAPE;
   if (batch * t > 0x7FFFFFFF || heads + 2 * kv_heads > 4096) return PLQ_ERR_LIMIT;
-  if (!qkv_bf16 || !cos_f32 || !sin_f32 || !q_out_bf16 || !k_cache_bf16 || !v_cache_bf16) return PLQ_ERR_NULL;
+  if (!qkv_bf16 || !cos_f32 || !sin_f32 || !q_out_bf16 || !k_cache || !v_cache) return PLQ_ERR_NULL;
   if (!aligned16(qkv_bf16) || !aligned16(cos_f32) || !aligned16(sin_f32) || !aligned16(q_out_bf16) ||
-      !aligned16(k_cache_bf16) || !aligned16(v_cache_bf16))
+      !aligned16(k_cache) || !aligned16(v_cache))
     return PLQ_ERR_ALIGN;
   int st = device_check();
   if (st != PLQ_OK) return st;
@@ -116,19 +229,67 @@ extern "C" int plq_rope_kv_append(const void* qkv_bf16, int64_t ld, const void* 
   a.cos = static_cast<const float*>(cos_f32);
   a.sin = static_cast<const float*>(sin_f32);
   a.q_out = static_cast<uint4*>(q_out_bf16);
-  a.k_dst = static_cast<uint4*>(k_cache_bf16);
-  a.v_dst = static_cast<uint4*>(v_cache_bf16);
+  a.k_dst = static_cast<uint4*>(k_cache);
+  a.v_dst = static_cast<uint4*>(v_cache);
   a.pos_dev = reinterpret_cast<const long long*>(pos_dev);
   a.pos = pos;
   a.t_max = t_max;
   a.status = dev_status;
   a.ld8 = ld / 8;
-  a.total = batch * t * (heads + 2 * kv_heads) * 8;
+  a.total = batch * t * (heads + 2 * kv_heads) * (packed ? 1 : 8);      // head rows, or threads
   a.t = static_cast<int>(t);
   a.heads = static_cast<int>(heads);
   a.kv_heads = static_cast<int>(kv_heads);
+  if (packed) {
+    rope_kv_append_nvfp4_kernel<<<static_cast<unsigned>((a.total + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
+    PLQ_CUDA_TRY(cudaGetLastError());
+    return PLQ_OK;
+  }
   const long long blocks = (a.total + 255) / 256;
   rope_kv_append_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  PLQ_CUDA_TRY(cudaGetLastError());
+  return PLQ_OK;
+}
+
+}  // namespace plq
+
+extern "C" int plq_rope_kv_append(const void* qkv_bf16, int64_t ld, const void* cos_f32, const void* sin_f32,
+                                  int64_t batch, int64_t t, int64_t heads, int64_t kv_heads, int64_t head_dim,
+                                  void* q_out_bf16, void* k_cache_bf16, void* v_cache_bf16, int64_t t_max,
+                                  const int64_t* pos_dev, int64_t pos, int32_t* dev_status, void* stream) {
+  return plq::launch_rope(false, qkv_bf16, ld, cos_f32, sin_f32, batch, t, heads, kv_heads, head_dim, q_out_bf16, k_cache_bf16,
+                          v_cache_bf16, t_max, pos_dev, pos, dev_status, stream);
+}
+
+extern "C" int plq_rope_kv_append_nvfp4(const void* qkv_bf16, int64_t ld, const void* cos_f32, const void* sin_f32,
+                                        int64_t batch, int64_t t, int64_t heads, int64_t kv_heads, int64_t head_dim,
+                                        void* q_out_bf16, void* k_cache, void* v_cache, int64_t t_max,
+                                        const int64_t* pos_dev, int64_t pos, int32_t* dev_status, void* stream) {
+  return plq::launch_rope(true, qkv_bf16, ld, cos_f32, sin_f32, batch, t, heads, kv_heads, head_dim, q_out_bf16, k_cache, v_cache,
+                          t_max, pos_dev, pos, dev_status, stream);
+}
+
+extern "C" int plq_unpack_head_rows(const void* k_rows, const void* v_rows, int64_t batch, int64_t t, int64_t t_max,
+                                    int64_t kv_heads, void* k_bf16, void* v_bf16, void* stream) {
+  using namespace plq;
+  if (batch < 0 || t < 0 || kv_heads < 1 || t > t_max) return PLQ_ERR_SHAPE;
+  if (batch * t > (1ll << 31) || kv_heads > 4096) return PLQ_ERR_LIMIT;
+  if (batch == 0 || t == 0) return PLQ_OK;
+  if (!k_rows || !v_rows || !k_bf16 || !v_bf16) return PLQ_ERR_NULL;
+  if (!aligned16(k_rows) || !aligned16(v_rows) || !aligned16(k_bf16) || !aligned16(v_bf16)) return PLQ_ERR_ALIGN;
+  int st = device_check();
+  if (st != PLQ_OK) return st;
+  UnpackRowsArgs a;
+  a.src[0] = static_cast<const uint8_t*>(k_rows);
+  a.src[1] = static_cast<const uint8_t*>(v_rows);
+  a.dst[0] = static_cast<uint4*>(k_bf16);
+  a.dst[1] = static_cast<uint4*>(v_bf16);
+  a.t_heads = t * kv_heads;
+  a.cap_heads = t_max * kv_heads;
+  a.total = batch * t * kv_heads * 16;
+  const long long blocks = (a.total + 255) / 256;
+  if (blocks > 0x7FFFFFFF) return PLQ_ERR_LIMIT;
+  unpack_head_rows_kernel<<<dim3(static_cast<unsigned>(blocks), 2, 1), 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
   PLQ_CUDA_TRY(cudaGetLastError());
   return PLQ_OK;
 }

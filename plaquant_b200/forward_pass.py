@@ -20,6 +20,7 @@ from __future__ import annotations
 
 import math
 import re
+import weakref
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Tuple
 
@@ -125,6 +126,7 @@ class ResQForwardB200:
                 self.lm_head = (torch.randn(c.vocab_size, c.hidden_size, generator=g, device=self.device) * 0.02).to(torch.bfloat16)
         self.kv: List[Tuple[torch.Tensor, torch.Tensor]] = []
         self.pos = 0
+        self._kv_room: List[Optional[tuple]] = []        # per layer: (weak references to the tensors of self.kv, rows allocated)
         self._decode_states: Dict[tuple, _DecodeState] = {}
         # keys go into the cache as NVFP4 (Hadamard over the head dimension, per-head rows), queries get the same
         # rotation: the reference's QKRotationWrapper with k_had (promix/quantize/kv_quant.py:244-279)
@@ -139,6 +141,9 @@ class ResQForwardB200:
         # packed rows in one kernel over peer memory instead of an NCCL all-reduce of bf16
         self.scatter = (tp.ScatterReduce(scatter_prefill_rows, c.hidden_size, self.k_hi_hidden, self.device, self.ctx.group)
                         if scatter_prefill_rows > 0 and self.ctx.size > 1 else None)
+
+    def __getstate__(self):
+        return {**self.__dict__, "_kv_room": []}         # weak references: a copy's first append copies its cache
 
     # ---- where the weights come from ---------------------------------------------------------------
     def _random_layer(self, li: int, seed: int) -> Dict[str, torch.Tensor]:
@@ -257,59 +262,95 @@ class ResQForwardB200:
         cache -> [B, T, heads * head_dim] (this rank's heads)."""
         c = self.cfg
         b, t, _ = qkv.shape
-        if not self.kv_quant and c.head_dim == 128:
-            # RoPE on q and k and the cache append in one kernel (same float32 arithmetic as _rope, bit for bit)
+        if c.head_dim == 128 and self.kv_quant != "fake":
+            # RoPE on q and k and the cache append in one kernel (the float32 arithmetic of _rope, bit for bit); into a
+            # packed cache it also rotates the keys and quantises (the bytes of kv_cache.pack_head_rows)
             cos, sin = cos_sin[0].reshape(t, c.head_dim), cos_sin[1].reshape(t, c.head_dim)
             if static is None:
-                k = torch.empty(b, t, self.kv_heads, c.head_dim, dtype=qkv.dtype, device=qkv.device)
-                v = torch.empty_like(k)
-                q = ops.rope_kv_append(qkv, cos, sin, self.heads, self.kv_heads, k, v, 0)
-                if pos0 == 0:
-                    self.kv[li] = (k, v)
-                else:
-                    self.kv[li] = (torch.cat([self.kv[li][0], k], 1), torch.cat([self.kv[li][1], v], 1))
-                kk, vv = self.kv[li]
-                attn = F.scaled_dot_product_attention(q.transpose(1, 2), kk.transpose(1, 2), vv.transpose(1, 2),
-                                                      is_causal=(t > 1), enable_gqa=True)
-            else:
-                kk, vv = static["k"][li], static["v"][li]
-                q = ops.rope_kv_append(qkv, cos, sin, self.heads, self.kv_heads, kk, vv, static["pos"])
-                attn = F.scaled_dot_product_attention(q.transpose(1, 2), kk.transpose(1, 2), vv.transpose(1, 2),
-                                                      attn_mask=static["mask"], enable_gqa=True)
-            return attn.transpose(1, 2).reshape(b, t, self.heads * c.head_dim)
+                k, v, n, cap = self._cache_room(li, b, t, pos0)
+                row = k.shape[2] * k.shape[3]
+                kk, vv = (x.as_strided((b, cap, *x.shape[2:]), (cap * row, row, x.shape[3], 1)) for x in (k, v))
+                q = ops.rope_kv_append(qkv, cos, sin, self.heads, self.kv_heads, kk, vv, n)
+                return self._attend(q, kk, vv, n + t, None)
+            kk, vv = static["k"][li], static["v"][li]
+            q = ops.rope_kv_append(qkv, cos, sin, self.heads, self.kv_heads, kk, vv, static["pos"])
+            return self._attend(q, kk, vv, kk.shape[1], static["mask"])
         q, k, v = qkv.split([self.heads * c.head_dim, self.kv_heads * c.head_dim, self.kv_heads * c.head_dim], -1)
         q, k, v = q.view(b, t, self.heads, c.head_dim), k.view(b, t, self.kv_heads, c.head_dim), v.view(b, t, self.kv_heads, c.head_dim)
         q, k = self._rope(q, k, cos_sin)
         if self.kv_quant:
-            # NVFP4 cache: keys rotated over the head dimension (queries get the same rotation), values as they are
-            # (the reference's k_bits / v_bits "nvfp4", promix/configs/llama-3-8b-mxfp8-nvfp4-kv4.yaml:20-25).  The
-            # cache holds the packed rows: 64 code bytes + 8 scale bytes per (token, head) instead of 256 bytes.
+            # keep, in bf16, exactly what the packed cache gives back
             q = kv_cache.rotate_heads(q)
-            k = kv_cache.pack_head_rows(k, hadamard=True)
-            v = kv_cache.pack_head_rows(v, hadamard=False)
-            if self.kv_quant == "fake":            # keep, in bf16, exactly what the packed cache gives back
-                k, v = kv_cache.unpack_head_rows(k), kv_cache.unpack_head_rows(v)
-        packed_cache = bool(self.kv_quant) and self.kv_quant != "fake"
+            k = kv_cache.unpack_head_rows(kv_cache.pack_head_rows(k, hadamard=True))
+            v = kv_cache.unpack_head_rows(kv_cache.pack_head_rows(v, hadamard=False))
         if static is None:
             if pos0 == 0:
                 self.kv[li] = (k, v)
             else:
                 self.kv[li] = (torch.cat([self.kv[li][0], k], 1), torch.cat([self.kv[li][1], v], 1))
             kk, vv = self.kv[li]
-            if packed_cache:                       # dequantise on read (no attention kernel reads the codes yet)
-                kk, vv = kv_cache.unpack_head_rows(kk), kv_cache.unpack_head_rows(vv)
             attn = F.scaled_dot_product_attention(q.transpose(1, 2), kk.transpose(1, 2), vv.transpose(1, 2),
                                                   is_causal=(t > 1), enable_gqa=True)
         else:
             kk, vv = static["k"][li], static["v"][li]
             kk.index_copy_(1, static["pos"], k)
             vv.index_copy_(1, static["pos"], v)
-            if packed_cache:
-                kk, vv = kv_cache.unpack_head_rows(kk), kv_cache.unpack_head_rows(vv)
             attn = F.scaled_dot_product_attention(q.transpose(1, 2), kk.transpose(1, 2), vv.transpose(1, 2),
                                                   attn_mask=static["mask"], enable_gqa=True)
         attn = attn.transpose(1, 2).reshape(b, t, self.heads * c.head_dim)
         return attn
+
+    def _attend(self, q: torch.Tensor, kk: torch.Tensor, vv: torch.Tensor, ctx: int, mask: Optional[torch.Tensor]) -> torch.Tensor:
+        """Queries [B, T, heads, 128] after RoPE over the first `ctx` positions of the caches (whole allocations)."""
+        b, t = q.shape[:2]
+        if self.kv_quant:
+            # NVFP4 cache: keys rotated over the head dimension (queries get the same rotation), values as they are
+            # (the reference's k_bits / v_bits "nvfp4", promix/configs/llama-3-8b-mxfp8-nvfp4-kv4.yaml:20-25).  The
+            # cache holds the packed rows: 64 code bytes + 8 scale bytes per (token, head) instead of 256 bytes;
+            # dequantised on read.
+            q = kv_cache.rotate_heads(q)
+            kk, vv = ops.unpack_head_rows(kk, vv, ctx)
+        elif ctx < kk.shape[1]:
+            kk, vv = kk[:, :ctx], vv[:, :ctx]
+        attn = F.scaled_dot_product_attention(q.transpose(1, 2), kk.transpose(1, 2), vv.transpose(1, 2), attn_mask=mask,
+                                              is_causal=(mask is None and t > 1), enable_gqa=True)
+        return attn.transpose(1, 2).reshape(b, t, self.heads * self.cfg.head_dim)
+
+    def _cache_room(self, li: int, b: int, t: int, pos0: int):
+        """Makes room for `t` more positions in the growing cache of layer `li`: `self.kv[li]` becomes the tensors that
+        include the new rows, still to be written.  Returns (keys, values, first new row, rows allocated): the two are
+        the leading positions of contiguous allocations.
+
+        Rows behind the views of `self.kv[li]` may be written in place only if these are the very tensors that the last
+        append made: then nobody else has a view of them.  Anything else - a prefill's cache, one restored from an
+        earlier step, one put there by the caller - is copied into a new allocation first, so every cache handed out
+        before keeps its contents."""
+        width, dtype = (kv_cache.ROW_BYTES, torch.uint8) if self.kv_quant else (kv_cache.HEAD_DIM, torch.bfloat16)
+        if len(self._kv_room) != len(self.layers):
+            self._kv_room = [None] * len(self.layers)
+        if pos0 == 0:                                # a prompt: exactly its own rows
+            new = tuple(torch.empty(b, t, self.kv_heads, width, dtype=dtype, device=self.device) for _ in range(2))
+            self.kv[li], self._kv_room[li] = new, None
+            return new[0], new[1], 0, t
+        k, v = self.kv[li]
+        n, room = k.shape[1], self._kv_room[li]
+        row = self.kv_heads * width
+        if room is not None and room[0]() is k and room[1]() is v and n + t <= room[2] and k.shape[0] == b:
+            cap = room[2]
+        else:
+            for old in (k, v):
+                if old.dtype != dtype or tuple(old.shape) != (b, n, self.kv_heads, width):
+                    raise RuntimeError(f"the cache of layer {li} is {old.dtype} {tuple(old.shape)}, the new rows need "
+                                       f"{dtype} {(b, n, self.kv_heads, width)}")
+            cap = n + t + min(256, max(32, n // 8))  # one copy in that many steps instead of one in each
+            new = [torch.empty(b, cap, self.kv_heads, width, dtype=dtype, device=self.device) for _ in range(2)]
+            new[0][:, :n].copy_(k)
+            new[1][:, :n].copy_(v)
+            k, v = new
+        size, stride = (b, n + t, self.kv_heads, width), (cap * row, row, width, 1)
+        k, v = self.kv[li] = k.as_strided(size, stride), v.as_strided(size, stride)
+        self._kv_room[li] = (weakref.ref(k), weakref.ref(v), cap)
+        return k, v, n, cap
 
     def _forward_layer(self, li: int, h: torch.Tensor, delta: Optional[torch.Tensor], pos0: int, cos_sin,
                        static: Optional[dict] = None):

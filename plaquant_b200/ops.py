@@ -228,8 +228,9 @@ def reduce_scatter_add_rmsnorm_pack(sr, rows_total: int, residual: torch.Tensor,
 def rope_kv_append(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, heads: int, kv_heads: int,
                    k_cache: torch.Tensor, v_cache: torch.Tensor, pos) -> torch.Tensor:
     """RoPE on the query and key heads of `qkv` (bf16 [B, T, (heads + 2 kv_heads) * 128]) and append of the rotated
-    keys and the values to `k_cache` / `v_cache` (bf16 [B, T_max, kv_heads, 128]) at positions pos .. pos + T - 1, one
-    kernel.  `cos` / `sin`: float32 with T * 128 elements (one row per new position).  `pos`: an int, or a device
+    keys and the values to `k_cache` / `v_cache` at positions pos .. pos + T - 1, one kernel.  The caches are bf16
+    [B, T_max, kv_heads, 128], or uint8 [B, T_max, kv_heads, 72]: rows as kv_cache.pack_head_rows makes them, keys
+    rotated by the Hadamard over the head dimension.  `cos` / `sin`: float32 with T * 128 elements (one row per new position).  `pos`: an int, or a device
     int64 tensor with one element (read by the kernel: a captured decode step appends at the current position).
     Returns the rotated queries, bf16 [B, T, heads, 128]."""
     _require_cuda(qkv, "qkv")
@@ -239,20 +240,39 @@ def rope_kv_append(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, head
     for name, c in (("cos", cos), ("sin", sin)):
         if c.dtype != torch.float32 or c.numel() != t * 128 or not c.is_contiguous():
             raise TypeError(f"{name} must be contiguous float32 with T * 128 elements")
-    t_max = k_cache.shape[1]
+    t_max, packed = k_cache.shape[1], k_cache.dtype == torch.uint8
+    want = (torch.uint8, 72) if packed else (torch.bfloat16, 128)
     for name, c in (("k_cache", k_cache), ("v_cache", v_cache)):
-        if c.dtype != torch.bfloat16 or not c.is_contiguous() or tuple(c.shape) != (b, t_max, kv_heads, 128):
-            raise TypeError(f"{name} must be contiguous bfloat16 [B, T_max, kv_heads, 128]")
+        if c.dtype != want[0] or not c.is_contiguous() or tuple(c.shape) != (b, t_max, kv_heads, want[1]):
+            raise TypeError(f"{name} must be contiguous bfloat16 [B, T_max, kv_heads, 128] or uint8 [B, T_max, kv_heads, 72]")
     on_device = isinstance(pos, torch.Tensor)
     if on_device and (pos.dtype != torch.int64 or pos.numel() != 1 or pos.device != qkv.device):
         raise TypeError("pos must be an int or a one-element int64 tensor on the device of qkv")
     q = torch.empty(b, t, heads, 128, dtype=torch.bfloat16, device=qkv.device)
     with torch.cuda.device(qkv.device):
-        st = _lib.lib().plq_rope_kv_append(_ptr(qkv), n, _ptr(cos), _ptr(sin), b, t, heads, kv_heads, 128, _ptr(q),
-                                           _ptr(k_cache), _ptr(v_cache), t_max, _ptr(pos) if on_device else None,
-                                           0 if on_device else int(pos), _ptr(status_word(qkv.device)), _stream(qkv.device))
+        fn = _lib.lib().plq_rope_kv_append_nvfp4 if packed else _lib.lib().plq_rope_kv_append
+        st = fn(_ptr(qkv), n, _ptr(cos), _ptr(sin), b, t, heads, kv_heads, 128, _ptr(q), _ptr(k_cache), _ptr(v_cache), t_max,
+                _ptr(pos) if on_device else None, 0 if on_device else int(pos), _ptr(status_word(qkv.device)),
+                _stream(qkv.device))
     _lib.check(st)
     return q
+
+
+def unpack_head_rows(k_rows: torch.Tensor, v_rows: torch.Tensor, t: int):
+    """bf16 values [B, t, kv_heads, 128] of the first `t` positions of two packed caches, contiguous uint8
+    [B, T_max, kv_heads, 72], in one launch."""
+    _require_cuda(k_rows, "k_rows")
+    b, t_max, kv_heads, width = k_rows.shape
+    for name, c in (("k_rows", k_rows), ("v_rows", v_rows)):
+        if c.dtype != torch.uint8 or not c.is_contiguous() or c.shape != k_rows.shape or width != 72 or c.device != k_rows.device:
+            raise TypeError(f"{name} must be contiguous uint8 [B, T_max, kv_heads, 72]")
+    k = torch.empty(b, t, kv_heads, 128, dtype=torch.bfloat16, device=k_rows.device)
+    v = torch.empty_like(k)
+    with torch.cuda.device(k_rows.device):
+        st = _lib.lib().plq_unpack_head_rows(_ptr(k_rows), _ptr(v_rows), b, t, t_max, kv_heads, _ptr(k), _ptr(v),
+                                             _stream(k_rows.device))
+    _lib.check(st)
+    return k, v
 
 
 def unpack(p: PackedMatrix) -> torch.Tensor:
