@@ -62,6 +62,25 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+_torch_lib = None
+
+
+def torch_lib():
+    """The library's PyTorch front end, _plq_torch.so.  Raises if it has not been built."""
+    global _torch_lib
+    if _torch_lib is None:
+        lib()
+        import torch  # noqa: F401  (the front end links against its libraries)
+        try:
+            from . import _plq_torch
+        except ImportError as e:
+            raise RuntimeError("_plq_torch.so is missing or does not load: build it with `python -m plaquant_b200.build` "
+                               "(there is no fallback path)") from e
+        _plq_torch.init(LIB_PATH)
+        _torch_lib = _plq_torch
+    return _torch_lib
+
+
 def check(status: int) -> None:
     if status != 0:
         text = lib().plq_status_string(status).decode()

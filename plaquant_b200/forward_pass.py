@@ -27,7 +27,7 @@ from typing import Dict, List, Optional, Tuple
 import torch
 import torch.nn.functional as F
 
-from . import kv_cache, ops, tp
+from . import _lib, kv_cache, ops, tp
 from .quantize import QuantizedLinear
 from .rotation import get_hadamard_matrix  # noqa: F401  (re-exported, as the reference module does)
 
@@ -68,6 +68,12 @@ class LlamaConfig:
     def llama3_8b(cls):
         return cls()
 
+
+# Up to this many rows a layer is one native call: there the host's time per launch bounds a pass (16 layers of hidden
+# size 4096, 333 rows: 4.9 ms operator by operator, 2.4 ms on the device).  Above it the kernels take several times longer
+# than their launches, and the operator path frees every intermediate as soon as it is consumed.
+NATIVE_LAYER_ROWS = 4096
+ROPE_TABLE_POSITIONS = 32768    # cos / sin rows made at construction (32 MB); later positions are computed per pass
 
 _IN_PEER_BUFFER = object()      # marker: a layer's MLP output is waiting, unreduced, in the peer buffer
 
@@ -133,6 +139,8 @@ class ResQForwardB200:
         self.kv_quant = kv_quant                     # False | True (packed NVFP4 rows in the cache) | "fake" (their bf16 values)
         if kv_quant and c.head_dim != 128:
             raise ValueError("kv_quant needs head_dim = 128 (one Hadamard block per head)")
+        self._rope_tables = self._rope_angles(torch.arange(ROPE_TABLE_POSITIONS, device=self.device, dtype=torch.float32))
+        torch.cuda.current_stream(self.device).synchronize()        # any stream may read them from here on
         # decode batches of up to `fused_reduce_rows` rows reduce over peer memory inside the RMSNorm-quant kernel
         self.peer = (tp.PeerReduce(fused_reduce_rows, c.hidden_size, self.device, self.ctx.group)
                      if fused_reduce_rows > 0 and self.ctx.size > 1 else None)
@@ -248,6 +256,12 @@ class ResQForwardB200:
         return (torch.cat([ang.cos(), ang.cos()], -1)[None, :, None, :],
                 torch.cat([ang.sin(), ang.sin()], -1)[None, :, None, :])
 
+    def _rope_rows(self, pos0, t: int):
+        """_rope_angles for the positions pos0 .. pos0 + t - 1 (the same values, from the tables where they reach)."""
+        if isinstance(pos0, int) and 0 <= pos0 and pos0 + t <= ROPE_TABLE_POSITIONS:
+            return tuple(x[:, pos0:pos0 + t] for x in self._rope_tables)
+        return self._rope_angles(torch.arange(pos0, pos0 + t, device=self.device, dtype=torch.float32))
+
     def _rope(self, q, k, cos_sin):
         c = self.cfg
         cos, sin = cos_sin
@@ -352,6 +366,38 @@ class ResQForwardB200:
         self._kv_room[li] = (weakref.ref(k), weakref.ref(v), cap)
         return k, v, n, cap
 
+    def _plain_layer(self, L: _Layer) -> bool:
+        """Is the layer made of this package's plain linears and norm weights (what the native call takes)?"""
+        for lin in (L.qkv, L.o, L.gate_up, L.down):
+            if type(lin) is not QuantizedLinear or not lin.online_had or lin.gemm_impl != "b200" or lin._gemm_w is None:
+                return False
+        for g in (L.ln1, L.ln2):
+            if g.dtype != torch.bfloat16 or g.numel() != self.cfg.hidden_size or not g.is_contiguous() or not g.is_cuda:
+                return False
+        return True
+
+    def _run_layers(self, h: torch.Tensor, pos0: int, cos_sin, static: Optional[dict] = None):
+        """All decoder layers: (residual stream, last MLP output not added to it yet)."""
+        delta, c = None, self.cfg
+        b, t, _ = h.shape
+        native = (self.ctx.size == 1 and c.head_dim == 128 and self.kv_quant != "fake" and 0 < b * t <= NATIVE_LAYER_ROWS
+                  and h.dtype == torch.bfloat16 and h.is_contiguous())
+        if native:
+            call, (cos, sin) = _lib.torch_lib().decoder_layer, cos_sin
+            had = kv_cache.head_rotation(h.device) if self.kv_quant else None
+        for li, L in enumerate(self.layers):
+            if not native or not self._plain_layer(L):
+                h, delta = self._forward_layer(li, h, delta, pos0, cos_sin, static=static)
+                continue
+            if static is None:
+                k, v, n, cap = self._cache_room(li, b, t, pos0)
+                pos_dev = mask = None
+            else:
+                k, v, n, cap, pos_dev, mask = static["k"][li], static["v"][li], 0, static["k"][li].shape[1], static["pos"], static["mask"]
+            h, delta = call(L.qkv.native(), L.o.native(), L.gate_up.native(), L.down.native(), L.ln1, L.ln2, self.heads,
+                            self.kv_heads, c.rms_eps, h, delta, cos, sin, k, v, cap, n, pos_dev, mask, had)
+        return h, delta
+
     def _forward_layer(self, li: int, h: torch.Tensor, delta: Optional[torch.Tensor], pos0: int, cos_sin,
                        static: Optional[dict] = None):
         """One decoder layer.  `h` is the residual stream and `delta` the previous layer's MLP output that has
@@ -410,10 +456,7 @@ class ResQForwardB200:
             self.kv = [None] * len(self.layers)
         h = F.embedding(input_ids, self.embed)
         t = input_ids.shape[1]
-        cos_sin = self._rope_angles(torch.arange(pos0, pos0 + t, device=h.device, dtype=torch.float32))   # once per pass
-        delta = None
-        for li in range(len(self.layers)):
-            h, delta = self._forward_layer(li, h, delta, pos0, cos_sin)
+        h, delta = self._run_layers(h, pos0, self._rope_rows(pos0, t))
         self.pos = pos0 + input_ids.shape[1]
         h = self._finish(h, delta)
         return self._logits(h if all_positions else h[:, -1])
@@ -512,9 +555,7 @@ class ResQForwardB200:
             st["mask"].copy_(torch.where(S.arange <= st["pos"], 0.0, float("-inf")).view(1, 1, 1, t_max))
             h = F.embedding(tok, self.embed)
             cos_sin = self._rope_angles(st["pos"].to(torch.float32))
-            delta = None
-            for li in range(len(self.layers)):
-                h, delta = self._forward_layer(li, h, delta, 0, cos_sin, static=st)
+            h, delta = self._run_layers(h, 0, cos_sin, static=st)
             tok.copy_(self._logits(self._finish(h, delta)[:, -1]).argmax(-1, keepdim=True))
             st["pos"].add_(1)
             step_idx.add_(1)

@@ -40,11 +40,16 @@ def dequantize_heads(p: ops.PackedMatrix, shape) -> torch.Tensor:
 def rotate_heads(q: torch.Tensor) -> torch.Tensor:
     """The same normalised Hadamard(128) on the head dimension of the queries (float32 product, one rounding:
     inference/quantize.py:447-448 in the reference)."""
-    key = (q.shape[-1], q.device)
+    return (q.float() @ head_rotation(q.device, q.shape[-1])).to(q.dtype)
+
+
+def head_rotation(device, size: int = 128) -> torch.Tensor:
+    """The normalised Hadamard matrix, float32, built once per device: no host-to-device copy inside a CUDA-graph capture."""
+    key = (size, torch.device(device))
     h = _H.get(key)
-    if h is None:                      # built once per device: no host-to-device copy inside a CUDA-graph capture
-        h = _H[key] = get_hadamard_matrix(q.shape[-1]).to(device=q.device, dtype=torch.float32)
-    return (q.float() @ h).to(q.dtype)
+    if h is None:
+        h = _H[key] = get_hadamard_matrix(size).to(device=device, dtype=torch.float32)
+    return h
 
 
 HEAD_DIM = 128

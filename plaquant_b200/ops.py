@@ -103,11 +103,14 @@ def pack(x: torch.Tensor, k_hi: int, hadamard: bool = False, sf_layout="tiled",
     if x.dtype != torch.bfloat16:
         raise TypeError("x must be bfloat16")
     k = x.shape[-1]
+    if out is None:
+        layout = _LAYOUTS[sf_layout]
+        bufs = _lib.torch_lib().pack(x, k_hi, hadamard, layout == SF_TILED, gamma, eps)
+        return PackedMatrix(x.numel() // k if k else 0, k - k_hi, k_hi, *bufs, layout)
     x2 = x.reshape(-1, k)
     if not x2.is_contiguous():
         x2 = x2.contiguous()
-    rows = x2.shape[0]
-    p = out if out is not None else alloc_packed(rows, k, k_hi, sf_layout, x.device, zero_padding=False)
+    rows, p = x2.shape[0], out
     L = _lib.lib()
     with torch.cuda.device(x.device):
         if gamma is None:
@@ -290,6 +293,11 @@ def _check_pair(a: PackedMatrix, b: PackedMatrix, layout: int) -> None:
         raise ValueError(f"K split mismatch: activations {a.k_lo}+{a.k_hi}, weights {b.k_lo}+{b.k_hi}")
     if a.sf_layout != layout or b.sf_layout != layout:
         raise ValueError("scale buffers are in the wrong layout for this kernel")
+
+
+def native_linear(w: PackedMatrix):
+    """The front end's object for a packed weight (tiled scales), complete before any call that uses it."""
+    return _lib.torch_lib().Linear(w.lo_codes, w.lo_sf, w.hi_codes, w.hi_sf, status_word(w.device), w.rows, w.k_lo, w.k_hi)
 
 
 GEMM_VARIANTS = {None: 0, "auto": 0, "128x128": 1, "128x256": 2, "pair256x256": 3}

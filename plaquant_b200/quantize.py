@@ -58,7 +58,7 @@ class QuantizedLinear:
         self.grouped, self.groupsize, self.clip_ratio = grouped, groupsize, clip_ratio
         self.online_had, self.had_matrix = online_had, had_matrix
         self.gemm_impl = "b200"
-        self._gemm_w = self._gemv_w = None
+        self._gemm_w = self._gemv_w = self._native = None
         if w_main_int.is_cuda:
             self._prepare()
 
@@ -95,9 +95,19 @@ class QuantizedLinear:
         self._gemm_w = ops.PackedMatrix(n, k_lo, k_hi, lo_c, _tile_sf(lo_s), hi_c,
                                         _tile_sf(hi_s) if k_hi else torch.zeros(0, dtype=torch.uint8, device=dev),
                                         ops.SF_TILED)
+        self._native = None
         # forward() declares the weights static (PLQ_GEMV_STATIC_B): the decode GEMV may then fetch them before the
         # kernels launched ahead of it have finished, so everything that produced them must be complete by now
         torch.cuda.current_stream(dev).synchronize()
+
+    def native(self):
+        """The packed weight as the front end's object, for the calls that take a whole linear or layer."""
+        if self._native is None:
+            self._native = ops.native_linear(self._gemm_w)
+        return self._native
+
+    def __getstate__(self):
+        return {**self.__dict__, "_native": None}       # made anew by the copy
 
     def to(self, device):
         self.w_main_int = self.w_main_int.to(device)
@@ -128,6 +138,10 @@ class QuantizedLinear:
             raise ValueError(f"Unknown gemm_impl: {self.gemm_impl}")
         if self._gemm_w is None:
             raise RuntimeError("QuantizedLinear weights are not on a CUDA device; call .to('cuda') (no CPU path)")
+        if isinstance(x, torch.Tensor):
+            y = self.native().forward(x, self.online_had, norm_weight, eps, out)
+            if y is not None:
+                return y
         if isinstance(x, ops.PackedMatrix):
             pa, lead = x, (x.rows,)
         else:

@@ -26,8 +26,10 @@ def init_kernel(path: Optional[str] = None, build_if_missing: bool = True):
     global _kernel_loaded
     if path is not None:
         _lib.LIB_PATH = path
-    elif build_if_missing and build.needs_build():
-        build.build_library()
+    elif build_if_missing:
+        if build.needs_build():
+            build.build_library()
+        build.build_torch_front_end()
     handle = _lib.lib()
     _kernel_loaded = True
     return handle

@@ -67,3 +67,13 @@ def test_no_gpu_means_arch_error_not_fallback(lib):
     import plaquant_b200 as plq
     with pytest.raises(RuntimeError):
         plq.pack(torch.zeros(1, 256, dtype=torch.bfloat16), 64)
+
+
+def test_torch_front_end_loads_and_leaves_cpu_tensors_to_the_caller(lib):
+    import torch
+    from plaquant_b200 import build, _lib
+    build.build_torch_front_end()
+    fe = _lib.torch_lib()
+    u8 = torch.zeros(0, dtype=torch.uint8)
+    lin = fe.Linear(u8, u8, u8, u8, torch.zeros(1, dtype=torch.int32), 8, 192, 64)
+    assert lin.forward(torch.zeros(1, 256, dtype=torch.bfloat16), False, None, 1e-6, None) is None

@@ -1,0 +1,78 @@
+"""The native calls that take a whole linear or half a decoder layer: the same kernels on the same operands as the
+operator-by-operator path, so every result is compared bit for bit with that path."""
+import copy
+import pickle
+
+import pytest
+import torch
+
+from tests._util import synth_activation, synth_weight
+
+pytestmark = pytest.mark.gpu
+plq = pytest.importorskip("plaquant_b200")
+
+
+# rows: one, the last of the decode kernel, the first of the GEMM, past one tile; k: scales padded (14336) or not
+@pytest.mark.parametrize("k,n,k_hi_fraction", [(4096, 384, 1 / 32), (14336, 256, 1 / 32), (1024, 264, 0.0)])
+@pytest.mark.parametrize("rows", [1, 16, 17, 130])
+def test_linear_call_equals_pack_and_product(rows, k, n, k_hi_fraction):
+    from plaquant_b200.quantize import QuantizedLinear
+    lin = QuantizedLinear.from_weight(synth_weight(n, k, seed=k + n).cuda(), high_fraction=k_hi_fraction)
+    x = synth_activation(rows, k, seed=rows).cuda()
+    gamma = (torch.rand(k, generator=torch.Generator().manual_seed(1)) + 0.5).to(torch.bfloat16).cuda()
+    for g in (None, gamma):
+        want = lin(lin.quantize_input(x, g))
+        got = lin(x, norm_weight=g)
+        assert torch.equal(got, want)
+    wide = torch.full((rows, n + 64), 7.0, dtype=torch.bfloat16, device="cuda")
+    lin(x, out=wide[:, 32:32 + n])
+    plain = lin(x)
+    assert torch.equal(wide[:, 32:32 + n], plain) and bool((wide[:, :32] == 7).all()) and bool((wide[:, 32 + n:] == 7).all())
+    strided = torch.zeros(rows, 2 * k, dtype=torch.bfloat16, device="cuda")[:, ::2]
+    strided.copy_(x)
+    assert torch.equal(lin(strided), plain) and torch.equal(lin(x.view(1, rows, 1, k)).view(rows, n), plain)
+    for other in (copy.deepcopy(lin), pickle.loads(pickle.dumps(lin))):
+        assert torch.equal(other(x), plain) and other.native() is not lin.native()
+    with pytest.raises(TypeError):
+        lin(x.float())
+    with pytest.raises(TypeError):
+        lin(x, norm_weight=gamma[:-1])
+    with pytest.raises((ValueError, plq.PlqError)):
+        lin(x[:, :-128].contiguous())
+    with pytest.raises(plq.PlqError):
+        lin(x[:0])
+    plq.check_device_status()
+
+
+@pytest.mark.parametrize("head_dim,heads,kv_heads,kv_quant", [(128, 4, 2, False), (128, 4, 1, True), (128, 4, 4, "fake"),
+                                                              (64, 4, 2, False), (128, 18, 2, False)])
+def test_layer_calls_equal_the_operator_path(monkeypatch, head_dim, heads, kv_heads, kv_quant):
+    """Prompt, a chunk behind it, single steps, graph decode; 18 heads over 2 key heads: no decode-attention kernel."""
+    from plaquant_b200 import forward_pass
+    cfg = forward_pass.LlamaConfig(hidden_size=heads * head_dim, intermediate_size=1024, num_layers=2, num_heads=heads,
+                                   num_kv_heads=kv_heads, head_dim=head_dim, vocab_size=400)
+    ids = torch.randint(0, 400, (3, 40), generator=torch.Generator().manual_seed(7)).cuda()
+    m = forward_pass.ResQForwardB200(cfg, "cuda", seed=3, kv_quant=kv_quant)
+
+    def everything():
+        out = [m.forward(ids[:, :21]), m.forward(ids[:, 21:24], pos0=21)]
+        out += [m.forward(ids[:, i:i + 1], pos0=i) for i in range(24, 28)]
+        out += [x.clone() for layer in m.kv for x in layer]
+        m._decode_states.clear()
+        return out + [m.generate(ids[:, :9], 5), m.forward(ids[:, :9], all_positions=True), m.forward(ids[:, :1])]
+    got = everything()
+    monkeypatch.setattr(forward_pass, "NATIVE_LAYER_ROWS", 0)
+    want = everything()
+    plq.check_device_status()
+    assert all(torch.equal(a, b) for a, b in zip(got, want)) and len(got) == len(want)
+
+
+def test_rope_rows_behind_the_table_equal_the_direct_form(monkeypatch):
+    from plaquant_b200 import forward_pass
+    cfg = forward_pass.LlamaConfig(hidden_size=256, intermediate_size=256, num_layers=1, num_heads=2, num_kv_heads=1,
+                                   head_dim=128, vocab_size=100)
+    m = forward_pass.ResQForwardB200(cfg, "cuda", seed=1)
+    for pos0, t in ((0, 1), (5, 7), (32767, 1), (32767, 2), (40000, 3)):
+        got = m._rope_rows(pos0, t)
+        want = m._rope_angles(torch.arange(pos0, pos0 + t, device="cuda", dtype=torch.float32))
+        assert all(a.shape == b.shape and torch.equal(a, b) for a, b in zip(got, want))
