@@ -243,6 +243,12 @@ PLQ_API int plq_gptq_block_frozen(const void* w_f32, int64_t ldw, const void* hi
                                   void* codes_u8, void* stream);
 
 /*
+ * Row-major scale bytes [rows, n_sf] -> PLQ_SF_TILED, plq_sf_tiled_bytes(rows, n_sf) bytes; padding rows and scales are
+ * zero.  The source may have any alignment.  Once per weight, when it is loaded (no reference counterpart: the reference has no tiled layout).
+ */
+PLQ_API int plq_tile_scales(const void* sf_rowmajor, void* sf_tiled, int64_t rows, int64_t n_sf, void* stream);
+
+/*
  * Dequantise a packed matrix back to bf16 [rows, k_lo + k_hi] (= the fake quantiser's return
  * value, promix/quantize/quant_utils.py:750-751, :706-707).
  */

@@ -927,33 +927,36 @@ extern "C" int plq_allreduce_add_rmsnorm_pack(const void* const* peer_x_dev, voi
 
 namespace plq {
 // Row-major scale bytes [rows, n_sf] -> the tiled layout the GEMM reads, one 32-bit word (four scales of one row)
-// per thread, consecutive threads writing consecutive words of a 512-byte chunk.  Scales beyond n_sf and rows beyond
+// per thread.  A warp takes eight neighbouring words of four rows: 32-byte pieces of the source, and 16-byte pieces of
+// eight chunks - the four rows r, r + 32, r + 64, r + 96 are consecutive words there.  Scales beyond n_sf and rows beyond
 // `rows` inside the last 128-row group are written as zero.
 __global__ void __launch_bounds__(256) tile_sf_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
-                                                      int rows, int n_sf, int chunks, long long words) {
-  const long long w = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (w >= words) return;
-  const int in_chunk = static_cast<int>(w & 127);             // (r & 31) * 4 + ((r >> 5) & 3)
-  const long long chunk_id = w >> 7;                           // (r >> 7) * chunks + kb / 4
-  const int c = static_cast<int>(chunk_id % chunks);
-  const int r = static_cast<int>(chunk_id / chunks) * 128 + (in_chunk & 3) * 32 + (in_chunk >> 2);
+                                                      int rows, int n_sf, int chunks) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = 8 * static_cast<int>(blockIdx.x) + (lane >> 2);                // chunk = four scales of the row
+  const int rq = 8 * static_cast<int>(blockIdx.y & 3) + warp;                  // row inside a quarter of the group
+  const int group = static_cast<int>(blockIdx.y >> 2);
+  if (c >= chunks) return;
+  const int r = group * 128 + (lane & 3) * 32 + rq;
   uint32_t v = 0;
   if (r < rows) {
     const uint8_t* p = src + static_cast<size_t>(r) * n_sf + 4 * c;
-    if (4 * c + 4 <= n_sf && (n_sf & 3) == 0) v = *reinterpret_cast<const uint32_t*>(p);
+    if (4 * c + 4 <= n_sf && ((static_cast<uintptr_t>(n_sf) | reinterpret_cast<uintptr_t>(src)) & 3) == 0) v = *reinterpret_cast<const uint32_t*>(p);
     else
       for (int i = 0; i < 4 && 4 * c + i < n_sf; ++i) v |= static_cast<uint32_t>(p[i]) << (8 * i);
   }
-  reinterpret_cast<uint32_t*>(dst)[w] = v;
+  reinterpret_cast<uint32_t*>(dst)[(static_cast<size_t>(group) * chunks + c) * 128 + 4 * rq + (lane & 3)] = v;
 }
 
 static int launch_tile_sf(const void* src, void* dst, int64_t rows, int64_t n_sf, cudaStream_t stream) {
-  if (n_sf == 0) return PLQ_OK;
-  const int64_t chunks = (n_sf + 3) / 4;
-  const long long words = ((rows + 127) / 128) * chunks * 128;
-  tile_sf_kernel<<<static_cast<unsigned>((words + 255) / 256), 256, 0, stream>>>(
-      static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), static_cast<int>(rows), static_cast<int>(n_sf),
-      static_cast<int>(chunks), words);
+  if (n_sf == 0 || rows == 0) return PLQ_OK;
+  const int64_t chunks = (n_sf + 3) / 4, groups = (rows + 127) / 128;
+  for (int64_t g0 = 0; g0 < groups; g0 += 16383) {             // four blocks of a group along y, at most 65535
+    const int64_t n = groups - g0 < 16383 ? groups - g0 : 16383;
+    tile_sf_kernel<<<dim3(static_cast<unsigned>((chunks + 7) / 8), static_cast<unsigned>(4 * n), 1), 256, 0, stream>>>(
+        static_cast<const uint8_t*>(src) + g0 * 128 * n_sf, static_cast<uint8_t*>(dst) + g0 * chunks * 512,
+        static_cast<int>(rows - g0 * 128), static_cast<int>(n_sf), static_cast<int>(chunks));
+  }
   return cudaGetLastError() == cudaSuccess ? PLQ_OK : PLQ_ERR_CUDA;
 }
 }  // namespace plq
@@ -983,6 +986,17 @@ extern "C" int plq_reduce_scatter_add_rmsnorm_pack(const void* const* peer_x_dev
   st = plq::launch_tile_sf(lo_sf_rowmajor, lo_sf_tiled, total_rows, (k - k_hi) / 16, cs);
   if (st == PLQ_OK) st = plq::launch_tile_sf(hi_sf_rowmajor, hi_sf_tiled, total_rows, k_hi / 32, cs);
   return st;
+}
+
+extern "C" int plq_tile_scales(const void* sf_rowmajor, void* sf_tiled, int64_t rows, int64_t n_sf, void* stream) {
+  using namespace plq;
+  if (rows < 0 || n_sf < 0) return PLQ_ERR_SHAPE;
+  if (rows > 0x7FFFFF00 || n_sf > (1 << 20)) return PLQ_ERR_LIMIT;
+  if (rows == 0 || n_sf == 0) return PLQ_OK;
+  if (!sf_rowmajor || !sf_tiled) return PLQ_ERR_NULL;
+  if (!aligned16(sf_tiled)) return PLQ_ERR_ALIGN;
+  const int st = device_check();
+  return st != PLQ_OK ? st : launch_tile_sf(sf_rowmajor, sf_tiled, rows, n_sf, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int plq_unpack(const void* lo_codes, const void* lo_sf, const void* hi_codes, const void* hi_sf,

@@ -278,6 +278,18 @@ def unpack_head_rows(k_rows: torch.Tensor, v_rows: torch.Tensor, t: int):
     return k, v
 
 
+def tile_scales(sf: torch.Tensor) -> torch.Tensor:
+    """Row-major scale bytes [rows, n] (contiguous, CUDA) -> the tiled layout, flat; padding is zero."""
+    _require_cuda(sf, "sf")
+    rows, n = sf.shape
+    sf = sf.to(torch.uint8)
+    L = _lib.lib()
+    out = torch.empty(L.plq_sf_tiled_bytes(rows, n), dtype=torch.uint8, device=sf.device)
+    with torch.cuda.device(sf.device):
+        _lib.check(L.plq_tile_scales(_ptr(sf), _ptr(out), rows, n, _stream(sf.device)))
+    return out
+
+
 def unpack(p: PackedMatrix) -> torch.Tensor:
     """Dequantise to bf16 [rows, K]: the value the reference's fake quantiser returns."""
     y = torch.empty(p.rows, p.k, dtype=torch.bfloat16, device=p.device)

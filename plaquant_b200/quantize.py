@@ -27,16 +27,6 @@ from . import ops, rotation
 SUPPORTED_FP_FORMATS = ("mxfp8", "nvfp4")
 
 
-def _tile_sf(sf: torch.Tensor) -> torch.Tensor:
-    """Row-major scale bytes [rows, n] -> the 128 x 4 tiled order (pure data movement, done once per weight)."""
-    rows, n = sf.shape
-    rp, npad = -(-rows // 128) * 128, -(-n // 4) * 4
-    full = torch.zeros(rp, npad, dtype=torch.uint8, device=sf.device)
-    full[:rows, :n] = sf
-    t = full.view(rp // 128, 4, 32, npad // 4, 4).permute(0, 3, 2, 1, 4)
-    return t.contiguous().view(-1)
-
-
 class QuantizedLinear:
     """One mixed NVFP4 / MXFP8 linear layer: y = x @ W^T with both operands quantised."""
 
@@ -92,8 +82,8 @@ class QuantizedLinear:
         hi_s = self.w_high_scale.contiguous() if k_hi else empty
         lo_c, lo_s = self.w_main_int.contiguous(), self.w_main_scale.contiguous()
         self._gemv_w = ops.PackedMatrix(n, k_lo, k_hi, lo_c, lo_s, hi_c, hi_s, ops.SF_ROWMAJOR)
-        self._gemm_w = ops.PackedMatrix(n, k_lo, k_hi, lo_c, _tile_sf(lo_s), hi_c,
-                                        _tile_sf(hi_s) if k_hi else torch.zeros(0, dtype=torch.uint8, device=dev),
+        self._gemm_w = ops.PackedMatrix(n, k_lo, k_hi, lo_c, ops.tile_scales(lo_s), hi_c,
+                                        ops.tile_scales(hi_s) if k_hi else torch.zeros(0, dtype=torch.uint8, device=dev),
                                         ops.SF_TILED)
         self._native = None
         # forward() declares the weights static (PLQ_GEMV_STATIC_B): the decode GEMV may then fetch them before the
