@@ -116,9 +116,10 @@ struct Linear {
   int64_t k() const { return k_lo + k_hi; }
   int64_t packed_bytes(int64_t rows) const { return PackedAt(nullptr, rows, k_lo, k_hi).bytes; }
 
-  int product(const PackedAt& a, int64_t rows, void* y, int64_t ldy, void* stream) const {
+  // `like`: the choice of kernel for another number of rows (the two sum K in different orders).
+  int product(const PackedAt& a, int64_t rows, void* y, int64_t ldy, void* stream, int64_t like = 0) const {
     int32_t* st = status.data_ptr<int32_t>();
-    if (rows <= 16)      // decode: stream the weights once
+    if (std::max(rows, like) <= 16)      // decode: stream the weights once
       return api.gemv_tc(a.lo, a.lo_sf, a.hi, a.hi_sf, ptr(lo), ptr(lo_sf), ptr(hi), ptr(hi_sf), rows, n, k_lo, k_hi, y, ldy, st,
                          PLQ_GEMV_STATIC_B, stream);
     return api.mixed_gemm(a.lo, a.lo_sf, a.hi, a.hi_sf, ptr(lo), ptr(lo_sf), ptr(hi), ptr(hi_sf), rows, n, k_lo, k_hi, y, ldy, st,
@@ -157,13 +158,14 @@ Tensor heads_first(const Tensor& t) { return t.transpose(1, 2); }
 // One decoder layer on one GPU: h + delta -> RMSNorm(ln1) -> qkv -> RoPE, cache append -> attention -> o_proj -> residual,
 // RMSNorm(ln2) -> gate_up -> SiLU * up -> down_proj.  Returns (residual stream, down_proj's output not added to it yet).
 // k_view / v_view: the first `ctx` positions of caches allocated for `cap`; the new rows go to `pos` (or *pos_dev).
-// Packed caches (uint8) need `had`, the float32 Hadamard of the queries.
+// Packed caches (uint8) need `had`, the float32 Hadamard of the queries.  With `last_only` everything behind the attention
+// runs for the last position of each sequence alone, results [B, 1, hidden] (the same bits: rows are independent).
 std::tuple<Tensor, Tensor> decoder_layer(const Linear& qkv, const Linear& o, const Linear& gate_up, const Linear& down,
                                          const Tensor& ln1, const Tensor& ln2, int64_t heads, int64_t kv_heads, double eps_,
                                          const Tensor& h, const std::optional<Tensor>& delta, const Tensor& cos,
                                          const Tensor& sin, const Tensor& k_view, const Tensor& v_view, int64_t cap, int64_t pos,
                                          const std::optional<Tensor>& pos_dev, const std::optional<Tensor>& mask,
-                                         const std::optional<Tensor>& had) {
+                                         const std::optional<Tensor>& had, bool last_only) {
   pybind11::gil_scoped_release nogil;
   const c10::cuda::CUDAGuard guard(h.device());
   const int64_t b = h.size(0), t = h.size(1), hidden = h.size(2), rows = b * t, ctx = k_view.size(1);
@@ -217,27 +219,33 @@ std::tuple<Tensor, Tensor> decoder_layer(const Linear& qkv, const Linear& o, con
     vv = at::empty_like(kk);
     check(api.unpack_head_rows(k_view.const_data_ptr(), v_view.const_data_ptr(), b, ctx, cap, kv_heads, kk.data_ptr(), vv.data_ptr(), stream));
   }
-  const Tensor attn = heads_first(at::scaled_dot_product_attention(heads_first(q), heads_first(kk), heads_first(vv), mask, 0.0,
+  Tensor attn = heads_first(at::scaled_dot_product_attention(heads_first(q), heads_first(kk), heads_first(vv), mask, 0.0,
                                                                    !mask && t > 1, std::nullopt, true))
                           .contiguous();
 
-  Tensor h2 = at::empty_like(h), delta2 = at::empty_like(h);
+  const int64_t like = rows;
+  if (last_only) {
+    attn = attn.slice(1, t - 1).contiguous();
+    h1 = h1.slice(1, t - 1).contiguous();
+  }
+  const int64_t out_rows = last_only ? b : rows;
+  Tensor h2 = at::empty_like(h1), delta2 = at::empty_like(h1);
   uint8_t* gu = act + out0;
   {
-    const PackedAt p(ws.data_ptr(), rows, o.k_lo, o.k_hi);
-    check(api.pack(attn.const_data_ptr(), rows, attn_width, o.k_hi, 1, p.lo, p.lo_sf, p.hi, p.hi_sf, PLQ_SF_TILED, stream));
-    check(o.product(p, rows, act, hidden, stream));
+    const PackedAt p(ws.data_ptr(), out_rows, o.k_lo, o.k_hi);
+    check(api.pack(attn.const_data_ptr(), out_rows, attn_width, o.k_hi, 1, p.lo, p.lo_sf, p.hi, p.hi_sf, PLQ_SF_TILED, stream));
+    check(o.product(p, out_rows, act, hidden, stream, like));
   }
   {
-    const PackedAt p(ws.data_ptr(), rows, gate_up.k_lo, gate_up.k_hi);
-    check(api.add_rmsnorm_pack(act, h1.const_data_ptr(), h2.data_ptr(), ln2.const_data_ptr(), eps, rows, hidden, gate_up.k_hi, 1, p.lo,
+    const PackedAt p(ws.data_ptr(), out_rows, gate_up.k_lo, gate_up.k_hi);
+    check(api.add_rmsnorm_pack(act, h1.const_data_ptr(), h2.data_ptr(), ln2.const_data_ptr(), eps, out_rows, hidden, gate_up.k_hi, 1, p.lo,
                                p.lo_sf, p.hi, p.hi_sf, PLQ_SF_TILED, stream));
-    check(gate_up.product(p, rows, gu, 2 * ffn, stream));
+    check(gate_up.product(p, out_rows, gu, 2 * ffn, stream, like));
   }
   {
-    const PackedAt p(ws.data_ptr(), rows, down.k_lo, down.k_hi);
-    check(api.silu_mul_pack(gu, gu + 2 * ffn, 2 * ffn, rows, ffn, down.k_hi, 1, p.lo, p.lo_sf, p.hi, p.hi_sf, PLQ_SF_TILED, stream));
-    check(down.product(p, rows, delta2.data_ptr(), hidden, stream));
+    const PackedAt p(ws.data_ptr(), out_rows, down.k_lo, down.k_hi);
+    check(api.silu_mul_pack(gu, gu + 2 * ffn, 2 * ffn, out_rows, ffn, down.k_hi, 1, p.lo, p.lo_sf, p.hi, p.hi_sf, PLQ_SF_TILED, stream));
+    check(down.product(p, out_rows, delta2.data_ptr(), hidden, stream, like));
   }
   return {h2, delta2};
 }

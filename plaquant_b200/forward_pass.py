@@ -376,8 +376,10 @@ class ResQForwardB200:
                 return False
         return True
 
-    def _run_layers(self, h: torch.Tensor, pos0: int, cos_sin, static: Optional[dict] = None):
-        """All decoder layers: (residual stream, last MLP output not added to it yet)."""
+    def _run_layers(self, h: torch.Tensor, pos0: int, cos_sin, static: Optional[dict] = None, last_only: bool = False):
+        """All decoder layers: (residual stream, last MLP output not added to it yet).  With `last_only` the caller reads
+        the last position of every sequence alone, and the result may hold just that one, [B, 1, hidden]: behind the last
+        layer's attention nothing reads the other rows, and o_proj, norms and the MLP work row by row."""
         delta, c = None, self.cfg
         b, t, _ = h.shape
         native = (self.ctx.size == 1 and c.head_dim == 128 and self.kv_quant != "fake" and 0 < b * t <= NATIVE_LAYER_ROWS
@@ -386,8 +388,10 @@ class ResQForwardB200:
             call, (cos, sin) = _lib.torch_lib().decoder_layer, cos_sin
             had = kv_cache.head_rotation(h.device) if self.kv_quant else None
         for li, L in enumerate(self.layers):
+            # prompts of up to 16 rows in all stay whole: the decode kernel's K split depends on the number of rows
+            tail = last_only and t > 1 and b * t > 16 and li + 1 == len(self.layers) and self.ctx.size == 1
             if not native or not self._plain_layer(L):
-                h, delta = self._forward_layer(li, h, delta, pos0, cos_sin, static=static)
+                h, delta = self._forward_layer(li, h, delta, pos0, cos_sin, static=static, last_only=tail and self._plain_layer(L))
                 continue
             if static is None:
                 k, v, n, cap = self._cache_room(li, b, t, pos0)
@@ -395,11 +399,11 @@ class ResQForwardB200:
             else:
                 k, v, n, cap, pos_dev, mask = static["k"][li], static["v"][li], 0, static["k"][li].shape[1], static["pos"], static["mask"]
             h, delta = call(L.qkv.native(), L.o.native(), L.gate_up.native(), L.down.native(), L.ln1, L.ln2, self.heads,
-                            self.kv_heads, c.rms_eps, h, delta, cos, sin, k, v, cap, n, pos_dev, mask, had)
+                            self.kv_heads, c.rms_eps, h, delta, cos, sin, k, v, cap, n, pos_dev, mask, had, tail)
         return h, delta
 
     def _forward_layer(self, li: int, h: torch.Tensor, delta: Optional[torch.Tensor], pos0: int, cos_sin,
-                       static: Optional[dict] = None):
+                       static: Optional[dict] = None, last_only: bool = False):
         """One decoder layer.  `h` is the residual stream and `delta` the previous layer's MLP output that has
         not been added to it yet (None for the first layer): the add is fused into this layer's first
         RMSNorm-quant kernel, and the layer returns its own (h, delta) in the same form.
@@ -420,6 +424,13 @@ class ResQForwardB200:
             h, pa = ops.add_rmsnorm_pack(delta, h, L.ln1, c.rms_eps, self.k_hi_hidden)
             qkv = L.qkv(pa).view(b, t, -1)
         attn = self._attention(li, qkv, pos0, cos_sin, static)
+        if last_only:
+            # the products stay on the kernel that the whole batch would run on (the two sum K in different orders)
+            h = h[:, -1:].contiguous()
+            o = ops.mixed_gemm(L.o.quantize_input(attn[:, -1]), L.o._gemm_w).view(h.shape)
+            h, pa = ops.add_rmsnorm_pack(o, h, L.ln2, c.rms_eps, self.k_hi_hidden)
+            pa = ops.silu_mul_pack(ops.mixed_gemm(pa, L.gate_up._gemm_w), self.k_hi_ffn)
+            return h, ops.mixed_gemm(pa, L.down._gemm_w).view(h.shape)
         if fused:
             L.o(attn.reshape(b * t, -1), out=self.peer.buffer(b * t))                   # partial sums stay in the peer buffer
             h, pa = ops.allreduce_add_rmsnorm_pack(self.peer, b * t, h, L.ln2, c.rms_eps, self.k_hi_hidden)
@@ -456,8 +467,10 @@ class ResQForwardB200:
             self.kv = [None] * len(self.layers)
         h = F.embedding(input_ids, self.embed)
         t = input_ids.shape[1]
-        h, delta = self._run_layers(h, pos0, self._rope_rows(pos0, t))
+        h, delta = self._run_layers(h, pos0, self._rope_rows(pos0, t), last_only=not all_positions)
         self.pos = pos0 + input_ids.shape[1]
+        if not all_positions and isinstance(delta, torch.Tensor):
+            h, delta = h[:, -1:], delta[:, -1:]
         h = self._finish(h, delta)
         return self._logits(h if all_positions else h[:, -1])
 

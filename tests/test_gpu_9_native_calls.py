@@ -76,3 +76,27 @@ def test_rope_rows_behind_the_table_equal_the_direct_form(monkeypatch):
         got = m._rope_rows(pos0, t)
         want = m._rope_angles(torch.arange(pos0, pos0 + t, device="cuda", dtype=torch.float32))
         assert all(a.shape == b.shape and torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("rows_limit", [0, 4096])
+@pytest.mark.parametrize("b,t,kv_quant", [(1, 17, False), (3, 40, False), (20, 3, True), (4, 4, False)])
+def test_last_position_logits_equal_those_of_every_position(monkeypatch, rows_limit, b, t, kv_quant):
+    """The layer behind the last attention runs for the last positions alone: logits and cache as of the whole pass."""
+    from plaquant_b200 import forward_pass
+    monkeypatch.setattr(forward_pass, "NATIVE_LAYER_ROWS", rows_limit)
+    cfg = forward_pass.LlamaConfig(hidden_size=512, intermediate_size=1024, num_layers=2, num_heads=4, num_kv_heads=2,
+                                   head_dim=128, vocab_size=400)
+    ids = torch.randint(0, 400, (b, t), generator=torch.Generator().manual_seed(t)).cuda()
+    m = forward_pass.ResQForwardB200(cfg, "cuda", seed=3, kv_quant=kv_quant)
+    last = m.forward(ids)
+    kv = [x for layer in m.kv for x in layer]
+    full = m.forward(ids, all_positions=True)
+    # the head's library GEMM may take another kernel for b rows than for b t: one bf16 step of a logit
+    assert (last - full[:, -1]).abs().max() <= 2.0 ** -7 * full[:, -1].abs().max()
+    assert all(torch.equal(x, y) for x, y in zip(kv, (x for layer in m.kv for x in layer)))
+    h = torch.nn.functional.embedding(ids, m.embed)
+    whole = m._run_layers(h, 0, m._rope_rows(0, t))
+    short = m._run_layers(h, 0, m._rope_rows(0, t), last_only=True)
+    assert all(torch.equal(x[:, -1], y[:, -1]) for x, y in zip(whole, short))
+    assert short[0].shape[1] == (1 if b * t > 16 else t)
+    plq.check_device_status()
