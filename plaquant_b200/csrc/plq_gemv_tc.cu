@@ -4,7 +4,7 @@
 // and the activations the N-side one (m rows, zero-filled to 16 by the TMA box), so the packed
 // NVFP4 / MXFP8 weight bytes go HBM -> shared memory (TMA) -> tensor core and no thread ever
 // touches, converts or scales them.  The kernel is bound by how fast the weight bytes stream in:
-// a ring of four 22 KiB stages (16 KiB of weight codes, 2 KiB of weight scales, 2 + 2 KiB of
+// a ring of four (a small grid: eight) 22 KiB stages (16 KiB of weight codes, 2 KiB of weight scales, 2 + 2 KiB of
 // activation codes and scales, which come from L2).  A CTA takes 104 KiB of shared memory so that two
 // CTAs share an SM: ~176 KiB per SM in flight, and the CTAs of the next launch can set up and prefetch
 // their weights while the previous launch's are still finishing.
@@ -40,8 +40,8 @@ constexpr int kGtN = 16;                                   // MMA N (activation 
 constexpr int kGtXBytes = kGtN * kStageKBytes;             // 2 KiB
 constexpr int kGtSfBytes = 4 * kSfChunk;                   // 2 KiB: four chunks of one 128-row group
 constexpr int kGtStageBytes = kABytes + kGtXBytes + 2 * kGtSfBytes;
-constexpr int kGtStagesAll = 4;                            // 4 x 22 KiB in flight per CTA; two CTAs share an SM
-template <int MR> constexpr int kGtStagesFor = kGtStagesAll;
+constexpr int kGtStagesShared = 4;                         // 4 x 22 KiB in flight per CTA; two CTAs share an SM
+constexpr int kGtStagesAlone = 8;                          // a launch of at most one CTA per SM
 constexpr uint32_t kGtProducers = 3;                         // warps 0, 2, 3: one thread each, stages round-robin
 constexpr int kGtAccStages = 2;
 constexpr int kGtAccCols = 32;                             // spacing of the two accumulators (16 used)
@@ -55,11 +55,12 @@ constexpr int kGtEpiThreads = 128;
 template <int MR> constexpr int kGtMaxSlicesFor = MR == 8 ? 4 : 3;
 constexpr int kGtMaxSlices = 4;
 template <int MR> constexpr int kGtSlotBytesFor = MR * 128 * 4;      // one partial: MR activation rows x 128 weight rows, float32
-template <int MR>
-constexpr size_t kGtSmemBytesFor = 1024 + static_cast<size_t>(kGtStagesFor<MR>) * kGtStageBytes + (kGtMaxSlicesFor<MR> - 1) * kGtSlotBytesFor<MR> + 512;
+template <int MR, int STAGES>
+constexpr size_t kGtSmemBytesFor = 1024 + static_cast<size_t>(STAGES) * kGtStageBytes + (kGtMaxSlicesFor<MR> - 1) * kGtSlotBytesFor<MR> + 512;
 static_assert(kGtSfCol0 + 2 * kGtSfSetCols <= kGtTmemCols, "tensor memory budget");
-static_assert(2 * (kGtSmemBytesFor<8> + 1024) <= 232448 && 2 * (kGtSmemBytesFor<16> + 1024) <= 232448,
+static_assert(2 * (kGtSmemBytesFor<8, kGtStagesShared> + 1024) <= 232448 && 2 * (kGtSmemBytesFor<16, kGtStagesShared> + 1024) <= 232448,
               "two CTAs per SM (1 KiB per CTA is reserved by the system)");
+static_assert(kGtSmemBytesFor<16, kGtStagesAlone> <= 232448, "one CTA per SM");
 
 struct GtMaps {
   CUtensorMap w_lo, x_lo, w_hi, x_hi, sfw_lo, sfx_lo, sfw_hi, sfx_hi;
@@ -105,9 +106,9 @@ __device__ __forceinline__ void st_cluster_f32(uint32_t cluster_addr, float v) {
 }
 
 // MR = 8 or 16: how many activation rows (accumulator columns) the epilogue handles.
-template <int MR>
+template <int MR, int STAGES>
 __global__ void __launch_bounds__(kGtThreads, 2) gemv_tc_kernel(const __grid_constant__ GtMaps maps, const GtArgs g) {
-  constexpr int kGtStages = kGtStagesFor<MR>;
+  constexpr int kGtStages = STAGES;
   constexpr int kGtSlotBytes = kGtSlotBytesFor<MR>;
   constexpr int kGtSlotFloats = MR * 128;
   extern __shared__ uint8_t smem_raw[];
@@ -383,21 +384,21 @@ static int g_gt_launch = 0;
 // ---- host side --------------------------------------------------------------------------------
 // How many clusters of each size the device can hold at once (one CTA per SM, clusters inside a GPC);
 // looked up once per thread and device.
-template <int MR>
+template <int MR, int STAGES>
 static int gt_max_clusters(int slices) {
   static thread_local int cached_dev = -1;
   static thread_local int table[kGtMaxSlices + 1];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   if (cached_dev != dev) {
-    if (cudaFuncSetAttribute(gemv_tc_kernel<MR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(kGtSmemBytesFor<MR>)) != cudaSuccess)
+    if (cudaFuncSetAttribute(gemv_tc_kernel<MR, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(kGtSmemBytesFor<MR, STAGES>)) != cudaSuccess)
       return 0;
     for (int s = 1; s <= kGtMaxSlicesFor<MR>; ++s) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(static_cast<unsigned>(s * 64), 1, 1);
       cfg.blockDim = dim3(kGtThreads, 1, 1);
-      cfg.dynamicSmemBytes = kGtSmemBytesFor<MR>;
+      cfg.dynamicSmemBytes = kGtSmemBytesFor<MR, STAGES>;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = static_cast<unsigned>(s);
@@ -406,7 +407,7 @@ static int gt_max_clusters(int slices) {
       cfg.attrs = attr;
       cfg.numAttrs = 1;
       int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, gemv_tc_kernel<MR>, &cfg) != cudaSuccess) n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, gemv_tc_kernel<MR, STAGES>, &cfg) != cudaSuccess) n = 0;
       table[s] = n;
     }
     (void)cudaGetLastError();
@@ -424,21 +425,18 @@ static void gt_plan(int64_t n, int64_t k_lo, int64_t k_hi, int sms, int* slices,
   int s = (2 * sms) / tiles;                           // two CTAs fit an SM
   if (s > kGtMaxSlicesFor<MR>) s = kGtMaxSlicesFor<MR>;
   if (s > k_stages) s = k_stages;
-  while (s > 1 && gt_max_clusters<MR>(s) < tiles) --s;
+  while (s > 1 && gt_max_clusters<MR, kGtStagesShared>(s) < tiles) --s;
   if (s < 1) s = 1;
   *slices = s;
   *grid = s > 1 ? tiles * s : (tiles < 2 * sms ? tiles : 2 * sms);      // two CTAs fit an SM
 }
 
-template <int MR>
-static int gt_launch(const GtMaps& tm, const GtArgs& g, int64_t n, int64_t k_lo, int64_t k_hi, cudaStream_t stream) {
-  int slices = 1, grid = 1;
-  if (gt_max_clusters<MR>(1) < 1) return PLQ_ERR_CUDA;     // also sets the kernel's shared-memory attribute
-  gt_plan<MR>(n, k_lo, k_hi, sm_count(), &slices, &grid);
+template <int MR, int STAGES>
+static int gt_launch_planned(const GtMaps& tm, const GtArgs& g, int slices, int grid, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
   cfg.blockDim = dim3(kGtThreads, 1, 1);
-  cfg.dynamicSmemBytes = kGtSmemBytesFor<MR>;
+  cfg.dynamicSmemBytes = kGtSmemBytesFor<MR, STAGES>;
   cfg.stream = stream;
   // Programmatic dependent launch: this kernel may start while the previous one in the stream drains; it
   // touches nothing that depends on earlier work before its griddepcontrol.wait.
@@ -451,8 +449,23 @@ static int gt_launch(const GtMaps& tm, const GtArgs& g, int64_t n, int64_t k_lo,
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  PLQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_tc_kernel<MR>, tm, g));
+  PLQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemv_tc_kernel<MR, STAGES>, tm, g));
   return PLQ_OK;
+}
+
+template <int MR>
+static int gt_launch(const GtMaps& tm, const GtArgs& g, int64_t n, int64_t k_lo, int64_t k_hi, cudaStream_t stream) {
+  int slices = 1, grid = 1;
+  if (gt_max_clusters<MR, kGtStagesShared>(1) < 1) return PLQ_ERR_CUDA;     // also sets the kernel's shared-memory attribute
+  gt_plan<MR>(n, k_lo, k_hi, sm_count(), &slices, &grid);
+  // A grid of at most one CTA per SM has the SM's shared memory to itself: a ring twice as deep, where a CTA has more
+  // stages than the shallow one holds (all clusters must still be resident at once).  Replayed alone, m = 16: 14336 -> 4096
+  // 11.5 -> 10.4 us, 4096 -> 6144 7.1 -> 6.6, m = 8: 4096 -> 4096 (five stages) 4.85 -> 5.5, the next GEMV losing its early
+  // start; between the other kernels of a decode step it is faster there too (16 layers, m = 2: 40.1 -> 39.3 ms in 16 steps).
+  const int64_t k_stages = g.lo_stages + g.hi_stages;
+  if (grid <= sm_count() && (k_stages + slices - 1) / slices > kGtStagesShared && gt_max_clusters<MR, kGtStagesAlone>(slices) * slices >= grid)
+    return gt_launch_planned<MR, kGtStagesAlone>(tm, g, slices, grid, stream);
+  return gt_launch_planned<MR, kGtStagesShared>(tm, g, slices, grid, stream);
 }
 
 }  // namespace plq
