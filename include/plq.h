@@ -214,6 +214,8 @@ PLQ_API int plq_rope_kv_append(const void* qkv_bf16, int64_t ld, const void* cos
  * plq_rope_kv_append into a packed NVFP4 cache, bytes [batch, t_max, kv_heads, 72]: per row 64 bytes of E2M1 codes and 8
  * E4M3 scale bytes, exactly what plq_pack(k_hi = 0, PLQ_SF_ROWMAJOR) makes of the row - with the Hadamard(128) for keys
  * (after RoPE), without it for values.  q_out holds the queries after RoPE, not rotated further.
+ * plq_rope_kv_append_nvfp4_values: both in one launch, over the first ctx positions (the new ones, inside them, included);
+ * q_out is float32, its values rounded to bf16.  With pos_dev, new rows at or behind position ctx are not reported as values.
  * plq_unpack_head_rows: the bf16 values [batch, t, kv_heads, 128] of the first t positions of two such caches (= plq_unpack).
  * Reference: promix/quantize/kv_quant.py:244-279.
  */
@@ -221,6 +223,11 @@ PLQ_API int plq_rope_kv_append_nvfp4(const void* qkv_bf16, int64_t ld, const voi
                                      int64_t batch, int64_t t, int64_t heads, int64_t kv_heads, int64_t head_dim,
                                      void* q_out_bf16, void* k_cache, void* v_cache, int64_t t_max,
                                      const int64_t* pos_dev, int64_t pos, int32_t* dev_status, void* stream);
+PLQ_API int plq_rope_kv_append_nvfp4_values(const void* qkv_bf16, int64_t ld, const void* cos_f32, const void* sin_f32,
+                                            int64_t batch, int64_t t, int64_t heads, int64_t kv_heads, int64_t head_dim,
+                                            void* q_out_f32, void* k_cache, void* v_cache, int64_t t_max,
+                                            const int64_t* pos_dev, int64_t pos, int64_t ctx, void* k_values_bf16,
+                                            void* v_values_bf16, int32_t* dev_status, void* stream);
 PLQ_API int plq_unpack_head_rows(const void* k_rows, const void* v_rows, int64_t batch, int64_t t, int64_t t_max,
                                  int64_t kv_heads, void* k_bf16, void* v_bf16, void* stream);
 

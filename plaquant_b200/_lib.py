@@ -33,6 +33,7 @@ SIGNATURES = {
                                                    _i64, _i64, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "plq_rope_kv_append": (_i32, [_vp, _i64, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _vp, _vp, _vp, _i64, _vp, _i64, _vp, _vp]),
     "plq_rope_kv_append_nvfp4": (_i32, [_vp, _i64, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _vp, _vp, _vp, _i64, _vp, _i64, _vp, _vp]),
+    "plq_rope_kv_append_nvfp4_values": (_i32, [_vp, _i64, _vp, _vp] + [_i64] * 5 + [_vp, _vp, _vp, _i64, _vp, _i64, _i64] + [_vp] * 4),
     "plq_unpack_head_rows": (_i32, [_vp, _vp, _i64, _i64, _i64, _i64, _vp, _vp, _vp]),
     "plq_gptq_block_frozen": (_i32, [_vp, _i64, _vp, _i64, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _vp, _i64, _vp, _vp, _vp]),
     "plq_gemv_tc": (_i32, [_vp] * 8 + [_i64] * 4 + [_vp, _i64, _vp, _i32, _vp]),

@@ -15,6 +15,14 @@ namespace plq {
 
 constexpr int kRopeHeadDim = 128;
 
+// Packed rows of keys and values -> their bf16 values.
+struct UnpackRowsArgs {
+  const uint8_t* src[2];     // [batch, t_max, kv_heads, 72]
+  uint4* dst[2];             // bf16 [batch, t, kv_heads, 128]
+  long long t_heads, cap_heads, total;     // t * kv_heads, t_max * kv_heads, threads per cache = batch * t * kv_heads * 16
+  int kv_heads;
+};
+
 struct RopeArgs {
   const uint4* qkv;        // bf16 [rows, ld]: [q heads | k heads | v heads] per row
   const float* cos;        // float32 [t, 128]: row tt belongs to position pos + tt
@@ -28,6 +36,11 @@ struct RopeArgs {
   long long ld8;           // row stride of qkv in 16-byte units
   long long total;         // rows * (heads + 2 kv_heads) * 8 threads
   int t, heads, kv_heads;
+  // packed cache only
+  UnpackRowsArgs old;      // the caches' bf16 values, or dst = nullptr
+  float2* q_f32;           // the queries as float32 (bf16-valued) instead of q_out
+  long long ctx;           // positions of `old`
+  unsigned append_blocks;
 };
 
 __device__ __forceinline__ void unpack_bf16x8(const uint4& q, float (&f)[8]) {
@@ -140,7 +153,15 @@ __device__ __forceinline__ HeadRow hadamard_row(HeadRow x, int lane) {
   return bf16_row(make_float2(__fmul_rn(__fadd_rn(x.a.x, x.b.x), c), __fmul_rn(__fadd_rn(x.a.y, x.b.y), c)),
                   make_float2(__fmul_rn(__fsub_rn(x.a.x, x.b.x), c), __fmul_rn(__fsub_rn(x.a.y, x.b.y), c)));
 }
-__device__ __forceinline__ void store_nvfp4_row(uint8_t* p, const HeadRow& x, int lane) {
+// Eight E2M1 codes times their scale -> four words of bf16 pairs: at most 7 significant bits, exact.
+__device__ __forceinline__ float e2m1_value(uint32_t c) {
+  const uint32_t mag = c & 7;
+  const float mv = mag < 2 ? 0.5f * mag : __uint_as_float(((mag >> 1) + 126u) << 23 | (mag & 1u) << 22);
+  return (c & 8) ? -mv : mv;
+}
+
+// Quantises the row into the cache and, where `values` is given, leaves there what the cache now holds.
+__device__ __forceinline__ void store_nvfp4_row(uint8_t* p, uint32_t* values, const HeadRow& x, int lane) {
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
     const float2 v = half ? x.b : x.a;
@@ -149,14 +170,53 @@ __device__ __forceinline__ void store_nvfp4_row(uint8_t* p, const HeadRow& x, in
     m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, 2));
     m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, 4));
     const uint32_t c = nvfp4_scale_code(m);
-    p[32 * half + lane] = static_cast<uint8_t>(nvfp4_quantize2(v, rcp_approx(e4m3_code_to_f32(c))));
+    const float s = e4m3_code_to_f32(c);
+    const uint32_t code = nvfp4_quantize2(v, rcp_approx(s));
+    p[32 * half + lane] = static_cast<uint8_t>(code);
+    if (values != nullptr) values[32 * half + lane] = pack_bf16x2(e2m1_value(code & 0xF) * s, e2m1_value(code >> 4) * s);
     if ((lane & 7) == 0) p[64 + 4 * half + (lane >> 3)] = static_cast<uint8_t>(c);
   }
 }
 
+// Packed rows of keys and values -> bf16, both caches, straight out of allocations with room for t_max positions: eight
+// elements (four code bytes, one scale byte) per thread, 16-byte stores.  Bound by the bytes written (256 per 72 read).
+// The positions [skip, skip + n_skip) are left to whoever appends them.
+__device__ __forceinline__ void unpack_rows(const UnpackRowsArgs& a, long long block, long long skip, int n_skip) {
+  const long long i = block * blockDim.x + threadIdx.x;
+  if (i >= 2 * a.total) return;
+  const bool value = i >= a.total;
+  const long long idx = value ? i - a.total : i;
+  const long long r = idx >> 4, b = r / a.t_heads, in_seq = r - b * a.t_heads;
+  if (n_skip != 0) {
+    const long long p = in_seq / a.kv_heads;
+    if (p >= skip && p < skip + n_skip) return;
+  }
+  const int j = static_cast<int>(idx & 15);
+  const uint8_t* p = (value ? a.src[1] : a.src[0]) + (b * a.cap_heads + in_seq) * kPackedRow;
+  const uint32_t codes = *reinterpret_cast<const uint32_t*>(p + 4 * j);
+  const float s = e4m3_code_to_f32(p[64 + (j >> 1)]);
+  uint32_t w[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) w[k] = pack_bf16x2(e2m1_value(codes >> (8 * k) & 0xF) * s, e2m1_value(codes >> (8 * k + 4) & 0xF) * s);
+  (value ? a.dst[1] : a.dst[0])[idx] = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+__global__ void __launch_bounds__(256) unpack_head_rows_kernel(const UnpackRowsArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  unpack_rows(a, blockIdx.x, 0, 0);
+}
+
+// One launch for a step over a packed cache: the first blocks rotate and append (and leave the new rows' values beside
+// the old ones'), the others dequantise the rows that were there.  As three launches - append, dequantisation, the
+// queries' widening to float32 - a decode step spent most of them waiting for the launch before.
 __global__ void __launch_bounds__(256) rope_kv_append_nvfp4_kernel(const RopeArgs a) {
   pdl_launch_dependents();
   pdl_wait();
+  if (blockIdx.x >= a.append_blocks) {             // the rows that were in the cache before
+    unpack_rows(a.old, blockIdx.x - a.append_blocks, (a.pos_dev != nullptr ? *a.pos_dev : a.pos), a.t);
+    return;
+  }
   const long long idx = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;      // head row
   if (idx >= a.total) return;
   const int lane = threadIdx.x & 31;
@@ -170,6 +230,12 @@ __global__ void __launch_bounds__(256) rope_kv_append_nvfp4_kernel(const RopeArg
   HeadRow x = {make_float2(bf16lo_to_f32(w0), bf16hi_to_f32(w0)), make_float2(bf16lo_to_f32(w1), bf16hi_to_f32(w1))};
   const bool is_q = head < a.heads, is_k = !is_q && head < a.heads + a.kv_heads;
   if (is_q || is_k) x = rope_row(x, a.cos + static_cast<size_t>(tt) * kRopeHeadDim, a.sin + static_cast<size_t>(tt) * kRopeHeadDim, lane);
+  if (is_q && a.q_f32 != nullptr) {
+    float2* dst = a.q_f32 + (row * a.heads + head) * 64 + lane;
+    dst[0] = x.a;
+    dst[32] = x.b;
+    return;
+  }
   if (is_q) {
     uint32_t* dst = reinterpret_cast<uint32_t*>(a.q_out + (row * a.heads + head) * 16) + lane;
     dst[0] = f32x2_to_bf16x2(x.a.x, x.a.y);
@@ -183,39 +249,12 @@ __global__ void __launch_bounds__(256) rope_kv_append_nvfp4_kernel(const RopeArg
   }
   if (is_k) x = hadamard_row(x, lane);
   const int kh = head - a.heads - (is_k ? 0 : a.kv_heads);
-  store_nvfp4_row(reinterpret_cast<uint8_t*>(is_k ? a.k_dst : a.v_dst) + ((b * a.t_max + p) * a.kv_heads + kh) * kPackedRow, x, lane);
+  uint4* values = is_k ? a.old.dst[0] : a.old.dst[1];
+  if (p >= a.ctx) values = nullptr;
+  if (values != nullptr) values += ((b * a.ctx + p) * a.kv_heads + kh) * 16;
+  store_nvfp4_row(reinterpret_cast<uint8_t*>(is_k ? a.k_dst : a.v_dst) + ((b * a.t_max + p) * a.kv_heads + kh) * kPackedRow,
+                  reinterpret_cast<uint32_t*>(values), x, lane);
 }
-
-// Packed rows of keys and values -> their bf16 values, both caches in one launch, straight out of caches with room for
-// t_max positions: eight elements (four code bytes, one scale byte) per thread, 16-byte stores.  A code times its scale
-// has at most 7 significant bits, so the bf16 value is exact (and equal to plq_unpack's).  Bound by the bytes written
-// (256 per 72 read).
-struct UnpackRowsArgs {
-  const uint8_t* src[2];     // [batch, t_max, kv_heads, 72]
-  uint4* dst[2];             // bf16 [batch, t, kv_heads, 128]
-  long long t_heads, cap_heads, total;     // t * kv_heads, t_max * kv_heads, threads per cache = batch * t * kv_heads * 16
-};
-
-__global__ void __launch_bounds__(256) unpack_head_rows_kernel(const UnpackRowsArgs a) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx >= a.total) return;
-  const long long r = idx >> 4, b = r / a.t_heads;
-  const int j = static_cast<int>(idx & 15);
-  const uint8_t* p = (blockIdx.y == 0 ? a.src[0] : a.src[1]) + (b * a.cap_heads + (r - b * a.t_heads)) * kPackedRow;
-  const uint32_t codes = *reinterpret_cast<const uint32_t*>(p + 4 * j);
-  const float s = e4m3_code_to_f32(p[64 + (j >> 1)]);
-  float f[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const uint32_t c = (codes >> (4 * i)) & 0xF, mag = c & 7;
-    const float mv = mag < 2 ? 0.5f * mag : __uint_as_float(((mag >> 1) + 126u) << 23 | (mag & 1u) << 22);
-    f[i] = (c & 8) ? -(mv * s) : mv * s;
-  }
-  (blockIdx.y == 0 ? a.dst[0] : a.dst[1])[idx] = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
-}
-
 
 template <typename Args>
 static int launch_overlapped(void (*kernel)(const Args), dim3 grid, const Args& a, void* stream) {
@@ -232,10 +271,26 @@ static int launch_overlapped(void (*kernel)(const Args), dim3 grid, const Args& 
   return PLQ_OK;
 }
 
+static UnpackRowsArgs unpack_args(const void* k_rows, const void* v_rows, int64_t batch, int64_t t, int64_t t_max, int64_t kv_heads,
+                                  void* k_bf16, void* v_bf16) {
+  UnpackRowsArgs a;
+  a.src[0] = static_cast<const uint8_t*>(k_rows);
+  a.src[1] = static_cast<const uint8_t*>(v_rows);
+  a.dst[0] = static_cast<uint4*>(k_bf16);
+  a.dst[1] = static_cast<uint4*>(v_bf16);
+  a.t_heads = t * kv_heads;
+  a.cap_heads = t_max * kv_heads;
+  a.total = batch * t * kv_heads * 16;
+  a.kv_heads = static_cast<int>(kv_heads);
+  return a;
+}
+
+// With `ctx` (packed cache): q_out is float32, and k_values / v_values receive the first ctx positions.
 static int launch_rope(bool packed, const void* qkv_bf16, int64_t ld, const void* cos_f32, const void* sin_f32,
                        int64_t batch, int64_t t, int64_t heads, int64_t kv_heads, int64_t head_dim,
                        void* q_out_bf16, void* k_cache, void* v_cache, int64_t t_max,
-                       const int64_t* pos_dev, int64_t pos, int32_t* dev_status, void* stream) {
+                       const int64_t* pos_dev, int64_t pos, int32_t* dev_status, void* stream, int64_t ctx = 0,
+                       void* k_values = nullptr, void* v_values = nullptr) {
   if (head_dim != kRopeHeadDim) return PLQ_ERR_SHAPE;
   if (batch < 1 || t < 1 || heads < 1 || kv_heads < 1 || t_max < 1) return PLQ_ERR_SHAPE;
   if (ld < (heads + 2 * kv_heads) * kRopeHeadDim || ld % 8 != 0) return PLQ_ERR_SHAPE;
@@ -263,7 +318,16 @@ static int launch_rope(bool packed, const void* qkv_bf16, int64_t ld, const void
   a.t = static_cast<int>(t);
   a.heads = static_cast<int>(heads);
   a.kv_heads = static_cast<int>(kv_heads);
-  if (packed) return launch_overlapped(rope_kv_append_nvfp4_kernel, dim3(static_cast<unsigned>((a.total + 7) / 8)), a, stream);
+  a.old = unpack_args(k_cache, v_cache, batch, ctx, t_max, kv_heads, k_values, v_values);
+  a.q_f32 = ctx > 0 ? static_cast<float2*>(q_out_bf16) : nullptr;
+  a.ctx = ctx;
+  a.append_blocks = static_cast<unsigned>((a.total + 7) / 8);
+  if (packed) {
+    // positions that are appended need no block of their own; a prompt has no others
+    const long long blocks = a.append_blocks + (ctx > t || (ctx > 0 && pos_dev) ? (2 * a.old.total + 255) / 256 : 0);
+    if (blocks > 0x7FFFFFFF) return PLQ_ERR_LIMIT;
+    return launch_overlapped(rope_kv_append_nvfp4_kernel, dim3(static_cast<unsigned>(blocks)), a, stream);
+  }
   return launch_overlapped(rope_kv_append_kernel, dim3(static_cast<unsigned>((a.total + 255) / 256)), a, stream);
 }
 
@@ -285,6 +349,20 @@ extern "C" int plq_rope_kv_append_nvfp4(const void* qkv_bf16, int64_t ld, const 
                           t_max, pos_dev, pos, dev_status, stream);
 }
 
+extern "C" int plq_rope_kv_append_nvfp4_values(const void* qkv_bf16, int64_t ld, const void* cos_f32, const void* sin_f32,
+                                               int64_t batch, int64_t t, int64_t heads, int64_t kv_heads, int64_t head_dim,
+                                               void* q_out_f32, void* k_cache, void* v_cache, int64_t t_max,
+                                               const int64_t* pos_dev, int64_t pos, int64_t ctx, void* k_values_bf16,
+                                               void* v_values_bf16, int32_t* dev_status, void* stream) {
+  using namespace plq;
+  if (ctx < t || ctx > t_max || (pos_dev == nullptr && pos + t > ctx)) return PLQ_ERR_SHAPE;
+  if (!k_values_bf16 || !v_values_bf16) return PLQ_ERR_NULL;
+  if (!aligned16(k_values_bf16) || !aligned16(v_values_bf16)) return PLQ_ERR_ALIGN;
+  if (batch * ctx > (1ll << 31)) return PLQ_ERR_LIMIT;
+  return launch_rope(true, qkv_bf16, ld, cos_f32, sin_f32, batch, t, heads, kv_heads, head_dim, q_out_f32, k_cache, v_cache, t_max,
+                     pos_dev, pos, dev_status, stream, ctx, k_values_bf16, v_values_bf16);
+}
+
 extern "C" int plq_unpack_head_rows(const void* k_rows, const void* v_rows, int64_t batch, int64_t t, int64_t t_max,
                                     int64_t kv_heads, void* k_bf16, void* v_bf16, void* stream) {
   using namespace plq;
@@ -295,15 +373,8 @@ extern "C" int plq_unpack_head_rows(const void* k_rows, const void* v_rows, int6
   if (!aligned16(k_rows) || !aligned16(v_rows) || !aligned16(k_bf16) || !aligned16(v_bf16)) return PLQ_ERR_ALIGN;
   int st = device_check();
   if (st != PLQ_OK) return st;
-  UnpackRowsArgs a;
-  a.src[0] = static_cast<const uint8_t*>(k_rows);
-  a.src[1] = static_cast<const uint8_t*>(v_rows);
-  a.dst[0] = static_cast<uint4*>(k_bf16);
-  a.dst[1] = static_cast<uint4*>(v_bf16);
-  a.t_heads = t * kv_heads;
-  a.cap_heads = t_max * kv_heads;
-  a.total = batch * t * kv_heads * 16;
-  const long long blocks = (a.total + 255) / 256;
+  const UnpackRowsArgs a = unpack_args(k_rows, v_rows, batch, t, t_max, kv_heads, k_bf16, v_bf16);
+  const long long blocks = (2 * a.total + 255) / 256;
   if (blocks > 0x7FFFFFFF) return PLQ_ERR_LIMIT;
-  return launch_overlapped(unpack_head_rows_kernel, dim3(static_cast<unsigned>(blocks), 2, 1), a, stream);
+  return launch_overlapped(unpack_head_rows_kernel, dim3(static_cast<unsigned>(blocks)), a, stream);
 }

@@ -27,8 +27,7 @@ struct Api {
   decltype(&::plq_gemv_tc) gemv_tc;
   decltype(&::plq_mixed_gemm) mixed_gemm;
   decltype(&::plq_rope_kv_append) rope_kv_append;
-  decltype(&::plq_rope_kv_append_nvfp4) rope_kv_append_nvfp4;
-  decltype(&::plq_unpack_head_rows) unpack_head_rows;
+  decltype(&::plq_rope_kv_append_nvfp4_values) rope_kv_append_nvfp4_values;
   decltype(&::plq_sf_tiled_bytes) sf_tiled_bytes;
 } api;
 
@@ -47,8 +46,7 @@ void init(const std::string& path) {
   find(api.gemv_tc, "plq_gemv_tc");
   find(api.mixed_gemm, "plq_mixed_gemm");
   find(api.rope_kv_append, "plq_rope_kv_append");
-  find(api.rope_kv_append_nvfp4, "plq_rope_kv_append_nvfp4");
-  find(api.unpack_head_rows, "plq_unpack_head_rows");
+  find(api.rope_kv_append_nvfp4_values, "plq_rope_kv_append_nvfp4_values");
   find(api.sf_tiled_bytes, "plq_sf_tiled_bytes");
 }
 
@@ -208,16 +206,18 @@ std::tuple<Tensor, Tensor> decoder_layer(const Linear& qkv, const Linear& o, con
     }
     check(qkv.product(p, rows, act, nq, stream));
   }
-  Tensor q = at::empty({b, t, heads, 128}, opts);
-  check((packed ? api.rope_kv_append_nvfp4 : api.rope_kv_append)(
-      act, nq, cos.const_data_ptr(), sin.const_data_ptr(), b, t, heads, kv_heads, 128, q.data_ptr(), k_view.data_ptr(), v_view.data_ptr(),
-      cap, pos_dev ? pos_dev->const_data_ptr<int64_t>() : nullptr, pos, status, stream));
-  Tensor kk = k_view, vv = v_view;
+  Tensor q = at::empty({b, t, heads, 128}, packed ? opts.dtype(at::kFloat) : opts), kk = k_view, vv = v_view;
+  const int64_t* at_pos = pos_dev ? pos_dev->const_data_ptr<int64_t>() : nullptr;
   if (packed) {
-    q = at::matmul(q.to(at::kFloat), *had).to(at::kBFloat16);
     kk = at::empty({b, ctx, kv_heads, 128}, opts);
     vv = at::empty_like(kk);
-    check(api.unpack_head_rows(k_view.const_data_ptr(), v_view.const_data_ptr(), b, ctx, cap, kv_heads, kk.data_ptr(), vv.data_ptr(), stream));
+    check(api.rope_kv_append_nvfp4_values(act, nq, cos.const_data_ptr(), sin.const_data_ptr(), b, t, heads, kv_heads, 128, q.data_ptr(),
+                                          k_view.data_ptr(), v_view.data_ptr(), cap, at_pos, pos, ctx, kk.data_ptr(), vv.data_ptr(),
+                                          status, stream));
+    q = at::matmul(q, *had).to(at::kBFloat16);
+  } else {
+    check(api.rope_kv_append(act, nq, cos.const_data_ptr(), sin.const_data_ptr(), b, t, heads, kv_heads, 128, q.data_ptr(),
+                             k_view.data_ptr(), v_view.data_ptr(), cap, at_pos, pos, status, stream));
   }
   Tensor attn = heads_first(at::scaled_dot_product_attention(heads_first(q), heads_first(kk), heads_first(vv), mask, 0.0,
                                                                    !mask && t > 1, std::nullopt, true))

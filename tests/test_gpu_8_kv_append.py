@@ -83,3 +83,31 @@ def test_decoder_steps_leave_earlier_caches_alone(kv_quant):
     with pytest.raises(RuntimeError):
         m.forward(ids[:, :1], pos0=60)                                 # a cache of another batch size
     plq.check_device_status()
+
+
+@pytest.mark.parametrize("b,t,heads,kv,pos,ctx,t_max", [(2, 1, 4, 2, 9, 10, 10), (3, 1, 8, 1, 0, 1, 16), (2, 5, 4, 2, 0, 5, 5),
+                                                       (1, 4, 6, 2, 30, 34, 60), (16, 1, 32, 8, 511, 512, 640), (2, 1, 2, 1, 5, 12, 12)])
+def test_append_with_values_equals_append_then_unpack(b, t, heads, kv, pos, ctx, t_max):
+    from plaquant_b200 import _lib, ops
+    g = torch.Generator().manual_seed(pos)
+    qkv = (torch.randn(b, t, (heads + 2 * kv) * 128, generator=g) * 2).to(torch.bfloat16).cuda()
+    cos, sin = (x.cuda() for x in _tables(pos, t))
+    rows = [torch.randint(0, 0x7F, (b, t_max, kv, 72), dtype=torch.uint8, generator=g).cuda() for _ in range(2)]
+    want_rows = [r.clone() for r in rows]
+    want_q = ops.rope_kv_append(qkv, cos, sin, heads, kv, *want_rows, pos)
+    want = ops.unpack_head_rows(*want_rows, ctx)
+    for at in (pos, torch.tensor([pos], device="cuda")):
+        if not isinstance(at, torch.Tensor) and pos + t > ctx:
+            continue
+        got_rows = [r.clone() for r in rows]
+        q = torch.empty(b, t, heads, 128, device="cuda")
+        vals = [torch.full((b, ctx, kv, 128), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+        on_device = isinstance(at, torch.Tensor)
+        _lib.check(_lib.lib().plq_rope_kv_append_nvfp4_values(
+            qkv.data_ptr(), qkv.shape[-1], cos.data_ptr(), sin.data_ptr(), b, t, heads, kv, 128, q.data_ptr(), got_rows[0].data_ptr(),
+            got_rows[1].data_ptr(), t_max, at.data_ptr() if on_device else None, 0 if on_device else at, ctx, vals[0].data_ptr(),
+            vals[1].data_ptr(), ops.status_word("cuda").data_ptr(), torch.cuda.current_stream().cuda_stream))
+        plq.check_device_status()
+        assert torch.equal(q, want_q.float())
+        assert all(torch.equal(x, y) for x, y in zip(got_rows, want_rows))
+        assert all(torch.equal(x.view(torch.int16), y.view(torch.int16)) for x, y in zip(vals, want))
