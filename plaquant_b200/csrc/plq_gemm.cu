@@ -78,6 +78,7 @@ struct GemmArgs {
   int lo_chunks, hi_chunks;        // scale chunks per 128-row group
   int wide_store;                  // y and ldy allow 32-byte stores
   int band;                        // row tiles per band of the tile order
+  int full_tiles;                  // tiles of full width; each one behind them is worked on as two of half the width
 };
 
 // Tile order: bands of `band` row tiles, inside a band M fastest, then N.  The CTAs that run at the same time
@@ -89,6 +90,22 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
   tn = r / rows;
   tm = b * band + (r - tn * rows);
 }
+
+// Work item `v` of a launch -> its row tile, first column and whether it is half a tile wide.  The items of a last wave
+// that would leave most of the CTA pairs idle are halved (256 x 128, one MMA of N = 128 per K step): 333 x 28672 has 224
+// tiles for 74 pairs, and the two left over after three waves cost a fourth of the time of a whole wave.
+template <int BN, int CG>
+struct WorkItem {
+  int tm, n0;
+  bool half;
+  __device__ __forceinline__ WorkItem(int v, const GemmArgs& g) {
+    half = CG == 2 && v >= g.full_tiles;
+    const int tile = half ? g.full_tiles + ((v - g.full_tiles) >> 1) : v;
+    int tn;
+    tile_coords(tile, g.tiles_m, g.tiles_n, g.band, tm, tn);
+    n0 = tn * BN + (half ? ((v - g.full_tiles) & 1) * (BN / 2) : 0);
+  }
+};
 
 template <int BN, int CG>
 __global__ void __launch_bounds__(GemmCfg<BN, CG>::kThreads, 1)
@@ -142,7 +159,7 @@ mixed_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs g) {
   const uint32_t tmem_base = *tmem_holder;
   pdl_launch_dependents();          // the next kernel in the stream may be launched while this one runs
 
-  const int num_tiles = g.tiles_m * g.tiles_n;
+  const int num_tiles = CG == 2 ? 2 * g.tiles_m * g.tiles_n - g.full_tiles : g.tiles_m * g.tiles_n;     // work items
   const int k_stages = g.lo_stages + g.hi_stages;
   const int first_tile = CG == 2 ? static_cast<int>(cluster_id_x()) : static_cast<int>(blockIdx.x);
   const int tile_step = CG == 2 ? static_cast<int>(nclusters_x()) : static_cast<int>(gridDim.x);
@@ -156,22 +173,25 @@ mixed_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs g) {
       // One stage's loads.  In a pair every load of both CTAs is counted on the leader's barrier, which is the
       // one the MMA issuer waits on; boxes always have their full size (out-of-range parts are zero-filled).
       auto issue = [&](uint32_t gs, int tile, int ks) {
-        int tm, tn;
-        tile_coords(tile, g.tiles_m, g.tiles_n, g.band, tm, tn);
-        const int mgrp = tm * CG + static_cast<int>(rank);        // this CTA's 128-row group of A
+        const WorkItem<BN, CG> w(tile, g);
+        const int mgrp = w.tm * CG + static_cast<int>(rank);      // this CTA's 128-row group of A
         const uint32_t slot = gs % C::kStages;
         const bool lo = ks < g.lo_stages;
         const int kk = lo ? ks : ks - g.lo_stages;
         const int chunk0 = lo ? kk * 4 : kk;              // NVFP4: one chunk per MMA; MXFP8: one per stage
         const uint32_t st = smem_base + slot * C::kStageBytes;
         const uint32_t bar = smem_u32(&full_bar[slot]) & (CG == 2 ? 0xFEFFFFFFu : 0xFFFFFFFFu);
-        if (leader) mbar_arrive_expect_tx(&full_bar[slot], CG * C::kStageBytes);
+        if (leader) mbar_arrive_expect_tx(&full_bar[slot], CG * (C::kStageBytes - (w.half ? C::kBBytes / 2 : 0)));
         tma_load_2d_cg<CG>(st, lo ? &tm_a_lo : &tm_a_hi, kk * kStageKBytes, mgrp * kBM, bar);
-        tma_load_2d_cg<CG>(st + kABytes, lo ? &tm_b_lo : &tm_b_hi, kk * kStageKBytes,
-                           tn * BN + static_cast<int>(rank) * C::kBRows, bar);
+        if (w.half)
+          tma_load_2d_cg<CG>(st + kABytes, lo ? &maps.b_lo_half : &maps.b_hi_half, kk * kStageKBytes,
+                             w.n0 + static_cast<int>(rank) * (C::kBRows / 2), bar);
+        else
+          tma_load_2d_cg<CG>(st + kABytes, lo ? &tm_b_lo : &tm_b_hi, kk * kStageKBytes,
+                             w.n0 + static_cast<int>(rank) * C::kBRows, bar);
         tma_load_3d_cg<CG>(st + kABytes + C::kBBytes, lo ? &maps.sfa_lo : &maps.sfa_hi, 0, chunk0, mgrp, bar);
         tma_load_3d_cg<CG>(st + kABytes + C::kBBytes + C::kSfaBytes, lo ? &maps.sfb_lo : &maps.sfb_hi, 0, chunk0,
-                           tn * C::kSfGroups, bar);
+                           w.n0 / 128, bar);
       };
       // Stage gs (running over all tiles of this CTA) belongs to producer gs % 2.  Both operands may have been
       // written by the kernel just before this one (a weight packed right before its first use included), so
@@ -197,8 +217,9 @@ mixed_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs g) {
     const bool elected = elect_one();
     if (elected && leader) {
       // ================================ MMA issuer ================================
-      constexpr uint32_t idesc_lo = make_idesc(1u /*E2M1*/, 128u * CG, BN, 0u /*UE4M3*/);
-      constexpr uint32_t idesc_hi = make_idesc(0u /*E4M3*/, 128u * CG, BN, 1u /*UE8M0*/);
+      constexpr uint32_t idesc_lo_full = make_idesc(1u /*E2M1*/, 128u * CG, BN, 0u /*UE4M3*/);
+      constexpr uint32_t idesc_hi_full = make_idesc(0u /*E4M3*/, 128u * CG, BN, 1u /*UE8M0*/);
+      constexpr uint32_t kIdescHalf = (BN / 2) >> 3 << 17;       // what the N field of half a tile is short of
       // barrier addresses to commit to: own CTA and, for a pair, the same barrier in the peer
       const uint32_t peer_off = CG == 2 ? map_to_cta(smem_u32(full_bar), 1u) - smem_u32(full_bar) : 0u;
       auto commit_all = [&](uint64_t* bar) {
@@ -218,6 +239,8 @@ mixed_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs g) {
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + as * BN;
+        const bool half = CG == 2 && tile >= g.full_tiles;
+        const uint32_t idesc_lo = idesc_lo_full - (half ? kIdescHalf : 0u), idesc_hi = idesc_hi_full - (half ? kIdescHalf : 0u);
         uint32_t accumulate = 0;
         for (int ks = 0; ks < k_stages; ++ks) {
             ok = CG == 2 ? mbar_wait_bounded_cluster(&full_bar[s], phase, abort_flag)
@@ -297,10 +320,9 @@ mixed_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs g) {
     bool ok = true;
     pdl_wait();                                       // the output may still be read by an earlier kernel
     for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
-      int tm, tn;
-      tile_coords(tile, g.tiles_m, g.tiles_n, g.band, tm, tn);
-      const int row = (tm * CG + static_cast<int>(rank)) * kBM + quad * 32 + lane;
-      const int col0 = tn * BN + cgp * C::kColsPerEpiWarp;
+      const WorkItem<BN, CG> w(tile, g);
+      const int row = (w.tm * CG + static_cast<int>(rank)) * kBM + quad * 32 + lane;
+      const int col0 = w.n0 + cgp * C::kColsPerEpiWarp;
       ok = mbar_wait_bounded_warp(&acc_full[as], aphase, abort_flag);
       if (!ok) break;
       tc_fence_after();
@@ -314,7 +336,7 @@ mixed_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs g) {
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(empty_addr + 8u * as);   // drained: the next tile may start
       if (++as == C::kAccStages) { as = 0; aphase ^= 1; }
-      if (row < g.m) {
+      if (row < g.m && !(w.half && cgp != 0)) {
         // Streaming stores (the output is written once and not read by this kernel: keep L2 for the
         // operands), 32 bytes = one full sector per thread and instruction when the row allows it.
         __nv_bfloat16* yrow = g.y + static_cast<size_t>(row) * g.ldy;
@@ -422,12 +444,14 @@ static int launch_gemm(const GemmPtrs& p, GemmArgs& g, cudaStream_t stream) {
   if (g.k_lo) {
     if ((st = make_tmap(&tm.a_lo, p.a_lo, g.m, g.k_lo / 2, kBM)) != PLQ_OK) return st;
     if ((st = make_tmap(&tm.b_lo, p.b_lo, g.n, g.k_lo / 2, C::kBRows)) != PLQ_OK) return st;
+    if (CG == 2 && (st = make_tmap(&tm.b_lo_half, p.b_lo, g.n, g.k_lo / 2, C::kBRows / 2)) != PLQ_OK) return st;
     if ((st = make_sf_tmap(&tm.sfa_lo, p.a_lo_sf, g.lo_chunks, mg, 1)) != PLQ_OK) return st;
     if ((st = make_sf_tmap(&tm.sfb_lo, p.b_lo_sf, g.lo_chunks, ng, C::kSfGroups)) != PLQ_OK) return st;
   }
   if (g.k_hi) {
     if ((st = make_tmap(&tm.a_hi, p.a_hi, g.m, g.k_hi, kBM)) != PLQ_OK) return st;
     if ((st = make_tmap(&tm.b_hi, p.b_hi, g.n, g.k_hi, C::kBRows)) != PLQ_OK) return st;
+    if (CG == 2 && (st = make_tmap(&tm.b_hi_half, p.b_hi, g.n, g.k_hi, C::kBRows / 2)) != PLQ_OK) return st;
     if ((st = make_sf_tmap(&tm.sfa_hi, p.a_hi_sf, g.hi_chunks, mg, 1)) != PLQ_OK) return st;
     if ((st = make_sf_tmap(&tm.sfb_hi, p.b_hi_sf, g.hi_chunks, ng, C::kSfGroups)) != PLQ_OK) return st;
   }
@@ -454,7 +478,11 @@ static int launch_gemm(const GemmPtrs& p, GemmArgs& g, cudaStream_t stream) {
   }
   const int tiles = g.tiles_m * g.tiles_n;
   const int slots = sm_count() / CG;                 // CTAs (CG = 1) or CTA pairs (CG = 2) resident at once
-  const int groups = tiles < slots ? tiles : slots;
+  // The last wave is halved where twice its tiles still fit one wave.
+  const int rest = tiles % slots;
+  g.full_tiles = CG == 2 && 2 * rest <= slots ? tiles - rest : tiles;
+  const int items = 2 * tiles - g.full_tiles;
+  const int groups = items < slots ? items : slots;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(groups * CG), 1, 1);
   cfg.blockDim = dim3(C::kThreads, 1, 1);
@@ -509,18 +537,20 @@ extern "C" int plq_mixed_gemm_variant(const void* a_lo_codes, const void* a_lo_s
   g.wide_store = (reinterpret_cast<uintptr_t>(y_bf16) % 32 == 0 && ldy % 16 == 0) ? 1 : 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (variant == PLQ_GEMM_AUTO) {
-    // The kernel is bound by the bytes a CTA pulls from L2 per K stage (38 KB for a CTA of a pair, 54 KB
-    // for a 128 x 256 tile, 36 KB for a 128 x 128 tile), so the cheapest shape is the one with the smallest
-    // (waves over the SMs) x (bytes per stage); ties go to the larger tile.
+    // The cheapest shape is the one with the smallest (waves over the SMs) x (time of a whole wave); ties go to the larger
+    // tile.  Times of a wave, measured on m = 8192 (K, N = 4096, 28672; 14336, 4096; 8192, 57344) and all within 3 %:
+    // pair 256 x 256 = 100, 128 x 256 = 120, 128 x 128 = 72, a wave of halved pair tiles = 80.  (The bytes per stage,
+    // 38 : 54 : 36 KB, had been the rule: it took the pair for 333 x 28672, 47 us against 40 - 44.)
     const int sms = sm_count();
     const int64_t mt = (m + 127) / 128;
     const int64_t pair_tiles = ((m + 255) / 256) * ((n + 255) / 256);
     const int64_t wide_tiles = mt * ((n + 255) / 256);
     const int64_t small_tiles = mt * ((n + 127) / 128);
     const int64_t pair_slots = sms / 2 > 0 ? sms / 2 : 1;
-    const int64_t cost_pair = ((pair_tiles + pair_slots - 1) / pair_slots) * 38;
-    const int64_t cost_wide = ((wide_tiles + sms - 1) / sms) * 54;
-    const int64_t cost_small = ((small_tiles + sms - 1) / sms) * 36;
+    const int64_t pair_rest = pair_tiles % pair_slots;            // a last wave of at most half the pairs runs halved
+    const int64_t cost_pair = pair_tiles / pair_slots * 100 + (pair_rest == 0 ? 0 : 2 * pair_rest <= pair_slots ? 80 : 100);
+    const int64_t cost_wide = ((wide_tiles + sms - 1) / sms) * 120;
+    const int64_t cost_small = ((small_tiles + sms - 1) / sms) * 72;
     variant = PLQ_GEMM_PAIR_256x256;
     int64_t best = cost_pair;
     if (cost_wide < best) { variant = PLQ_GEMM_128x256; best = cost_wide; }

@@ -17,6 +17,7 @@ constexpr int kSfChunk = 512;                     // one tiled scale chunk: 128 
 // scale buffers as 3-D int32 [128 words = one 512-byte chunk, chunks per group, 128-row groups].
 struct GemmMaps {
   CUtensorMap a_lo, b_lo, a_hi, b_hi, sfa_lo, sfb_lo, sfa_hi, sfb_hi;
+  CUtensorMap b_lo_half, b_hi_half;   // boxes of half the B rows, for the half-width tiles of the last wave
 };
 
 // Shared-memory matrix descriptors, split into a low word (address field, changes per stage) and a

@@ -178,3 +178,20 @@ def test_argument_errors():
     with pytest.raises(plq.PlqError) as e:
         plq.mixed_gemm(pa, pb)
     assert e.value.status == -2
+
+
+# A last wave of at most half the pairs is worked on in half tiles: a lone tile (all of it halved; n that ends in its first
+# half, at its edge, in its second half), rows past one CTA, whole waves with a few tiles left (74 pairs on 148 SMs: 76,
+# 150 and 224 tiles); k: ragged last stages of both formats, one format only, more stages than the ring
+@pytest.mark.parametrize("m,n,k,k_hi", [(1, 8, 128, 64), (77, 128, 1024, 64), (129, 136, 192, 64), (256, 256, 512, 128),
+                                        (300, 640, 384, 384), (333, 392, 14336, 448), (100, 19456, 256, 64), (300, 19208, 448, 0),
+                                        (333, 28672, 1024, 64)])
+def test_half_tiles_of_the_last_wave_equal_other_tile_shapes(m, n, k, k_hi):
+    x, w = synth_activation(m, k, seed=m + k).cuda(), synth_weight(n, k, seed=n + k + 1).cuda()
+    had = k % 128 == 0
+    pa, pb = (plq.pack(t, k_hi, hadamard=had, sf_layout="tiled") for t in (x, w))
+    y = _run(pa, pb, "pair256x256")
+    assert np.array_equal(y, _run(pa, pb, "128x128"))              # the same K order: the same bits
+    assert np.array_equal(y, _run(pa, pb, None))
+    if n < 1000:
+        assert rel_l2(y, _oracle_bf16(packed_to_numpy(pa), packed_to_numpy(pb))) <= TOL
