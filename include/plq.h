@@ -280,6 +280,16 @@ PLQ_API int plq_mixed_gemm(const void* a_lo_codes, const void* a_lo_sf, const vo
                    void* y_bf16, int64_t ldy, int32_t* dev_status, void* stream);
 
 /*
+ * y[m, n] = SiLU(gate) * up for the fused projection [gate | up] = A B^T, B of 2 n rows (n a multiple of 128), with the
+ * roundings to bf16 of plq_mixed_gemm followed by plq_silu_mul_pack's prologue: the products, SiLU, the result.
+ * Replaces gate_proj, up_proj and `silu(gate) * up` (inference/forward_pass.py:264-268).
+ */
+PLQ_API int plq_mixed_gemm_silu_mul(const void* a_lo_codes, const void* a_lo_sf, const void* a_hi_codes, const void* a_hi_sf,
+                                    const void* b_lo_codes, const void* b_lo_sf, const void* b_hi_codes, const void* b_hi_sf,
+                                    int64_t m, int64_t n, int64_t k_lo, int64_t k_hi, void* y_bf16, int64_t ldy,
+                                    int32_t* dev_status, void* stream);
+
+/*
  * plq_mixed_gemm with the tile shape chosen by the caller instead of by the built-in heuristic
  * (tests and tuning).  Same reference counterpart.
  */

@@ -21,6 +21,7 @@ SIGNATURES = {
     "plq_unpack": (_i32, [_vp, _vp, _vp, _vp, _i32, _i64, _i64, _i64, _vp, _vp]),
     "plq_tile_scales": (_i32, [_vp, _vp, _i64, _i64, _vp]),
     "plq_mixed_gemm": (_i32, [_vp] * 8 + [_i64] * 4 + [_vp, _i64, _vp, _vp]),
+    "plq_mixed_gemm_silu_mul": (_i32, [_vp] * 8 + [_i64] * 4 + [_vp, _i64, _vp, _vp]),
     "plq_mixed_gemm_variant": (_i32, [_vp] * 8 + [_i64] * 4 + [_vp, _i64, _vp, _vp, _i32]),
     "plq_gemv_workspace_bytes": (_i64, [_i64]),
     "plq_gemv": (_i32, [_vp] * 8 + [_i64] * 4 + [_vp, _i64, _vp, _i64, _vp]),

@@ -37,6 +37,7 @@
 #include <cuda.h>
 #include <cstring>
 
+#include "plq_quant.cuh"
 #include "plq_tc.cuh"
 
 namespace plq {
@@ -78,6 +79,7 @@ struct GemmArgs {
   int lo_chunks, hi_chunks;        // scale chunks per 128-row group
   int wide_store;                  // y and ldy allow 32-byte stores
   int band;                        // row tiles per band of the tile order
+  int up_row;                      // gated form: first "up" row of B (= n, the width of the output)
   int full_tiles;                  // tiles of full width; each one behind them is worked on as two of half the width
 };
 
@@ -107,10 +109,16 @@ struct WorkItem {
   }
 };
 
-template <int BN, int CG>
+// GATED: B holds [gate | up] rows and the output is SiLU(gate) * up, rounded to bf16 where the three operators it replaces
+// round (the products, the activation, their product).  A tile is 128 gate columns beside the 128 up columns they meet:
+// in a pair one CTA's half of B each.  The [m, 2 n] intermediate is neither written nor read back: at 8192 x 2 x 14336
+// that is half of the GEMM's stores and half of the loads of the pack kernel that follows.
+template <int BN, int CG, bool GATED>
 __global__ void __launch_bounds__(GemmCfg<BN, CG>::kThreads, 1)
 mixed_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs g) {
   using C = GemmCfg<BN, CG>;
+  static_assert(!GATED || BN == 256, "gated tiles are 128 + 128 columns");
+  constexpr int kOutN = GATED ? BN / 2 : BN;         // output columns of a tile
   const CUtensorMap& tm_a_lo = maps.a_lo;  const CUtensorMap& tm_b_lo = maps.b_lo;
   const CUtensorMap& tm_a_hi = maps.a_hi;  const CUtensorMap& tm_b_hi = maps.b_hi;
   extern __shared__ uint8_t smem_raw[];
@@ -183,6 +191,22 @@ mixed_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs g) {
         const uint32_t bar = smem_u32(&full_bar[slot]) & (CG == 2 ? 0xFEFFFFFFu : 0xFFFFFFFFu);
         if (leader) mbar_arrive_expect_tx(&full_bar[slot], CG * (C::kStageBytes - (w.half ? C::kBBytes / 2 : 0)));
         tma_load_2d_cg<CG>(st, lo ? &tm_a_lo : &tm_a_hi, kk * kStageKBytes, mgrp * kBM, bar);
+        if constexpr (GATED) {
+          const int col = w.n0 / 2;                       // gate columns col .. col + 127 and the up columns beside them
+          const CUtensorMap* tm_b = lo ? &tm_b_lo : &tm_b_hi;                 // boxes of 128 rows
+          const CUtensorMap* tm_sf = lo ? &maps.sfb_lo : &maps.sfb_hi;         // boxes of one 128-row group
+          const uint32_t sfb = st + kABytes + C::kBBytes + C::kSfaBytes;
+          if constexpr (CG == 2) {
+            tma_load_2d_cg<CG>(st + kABytes, tm_b, kk * kStageKBytes, (leader ? 0 : g.up_row) + col, bar);
+          } else {
+            tma_load_2d_cg<CG>(st + kABytes, tm_b, kk * kStageKBytes, col, bar);
+            tma_load_2d_cg<CG>(st + kABytes + C::kBBytes / 2, tm_b, kk * kStageKBytes, g.up_row + col, bar);
+          }
+          tma_load_3d_cg<CG>(st + kABytes + C::kBBytes, lo ? &maps.sfa_lo : &maps.sfa_hi, 0, chunk0, mgrp, bar);
+          tma_load_3d_cg<CG>(sfb, tm_sf, 0, chunk0, col / 128, bar);
+          tma_load_3d_cg<CG>(sfb + C::kSfbBytes / 2, tm_sf, 0, chunk0, (g.up_row + col) / 128, bar);
+          return;
+        }
         if (w.half)
           tma_load_2d_cg<CG>(st + kABytes, lo ? &maps.b_lo_half : &maps.b_hi_half, kk * kStageKBytes,
                              w.n0 + static_cast<int>(rank) * (C::kBRows / 2), bar);
@@ -322,15 +346,17 @@ mixed_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs g) {
     for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
       const WorkItem<BN, CG> w(tile, g);
       const int row = (w.tm * CG + static_cast<int>(rank)) * kBM + quad * 32 + lane;
-      const int col0 = w.n0 + cgp * C::kColsPerEpiWarp;
+      const int col0 = (GATED ? w.n0 / 2 + cgp * (C::kColsPerEpiWarp / 2) : w.n0 + cgp * C::kColsPerEpiWarp);
       ok = mbar_wait_bounded_warp(&acc_full[as], aphase, abort_flag);
       if (!ok) break;
       tc_fence_after();
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + as * BN + cgp * C::kColsPerEpiWarp;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + as * BN +
+                             cgp * (GATED ? C::kColsPerEpiWarp / 2 : C::kColsPerEpiWarp);
       // all loads first, one wait: the accumulator is handed back after a single tensor-memory round trip
       uint32_t r[C::kColsPerEpiWarp / 32][32];
 #pragma unroll
-      for (int c = 0; c < C::kColsPerEpiWarp / 32; ++c) tc_ld_32x32b_x32(taddr + c * 32, r[c]);
+      for (int c = 0; c < C::kColsPerEpiWarp / 32; ++c)      // gated: 64 gate columns, then the 64 up columns beside them
+        tc_ld_32x32b_x32(taddr + (GATED && c >= 2 ? kOutN - 64 : 0) + c * 32, r[c]);
       tc_wait_ld();
       tc_fence_before();
       __syncwarp();
@@ -342,12 +368,20 @@ mixed_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs g) {
         __nv_bfloat16* yrow = g.y + static_cast<size_t>(row) * g.ldy;
         const bool wide = g.wide_store;
 #pragma unroll
-        for (int v = 0; v < C::kColsPerEpiWarp / 16; ++v) {
+        for (int v = 0; v < C::kColsPerEpiWarp / (GATED ? 32 : 16); ++v) {
           const int col = col0 + v * 16;
           uint32_t d[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const int cc = v * 16 + 2 * i;
+            if constexpr (GATED) {
+              const uint32_t gate = f32x2_to_bf16x2(__uint_as_float(r[cc >> 5][cc & 31]), __uint_as_float(r[cc >> 5][(cc & 31) + 1]));
+              const uint32_t up = f32x2_to_bf16x2(__uint_as_float(r[2 + (cc >> 5)][cc & 31]), __uint_as_float(r[2 + (cc >> 5)][(cc & 31) + 1]));
+              const float2 sl = silu2(make_float2(bf16lo_to_f32(gate), bf16hi_to_f32(gate)));
+              const uint32_t act = f32x2_to_bf16x2(sl.x, sl.y);
+              const float2 prod = __fmul2_rn(make_float2(bf16lo_to_f32(act), bf16hi_to_f32(act)), make_float2(bf16lo_to_f32(up), bf16hi_to_f32(up)));
+              d[i] = f32x2_to_bf16x2(prod.x, prod.y);
+            } else
             asm("cvt.rn.bf16x2.f32 %0, %1, %2;"
                 : "=r"(d[i])
                 : "f"(__uint_as_float(r[cc >> 5][(cc & 31) + 1])), "f"(__uint_as_float(r[cc >> 5][cc & 31])));
@@ -434,40 +468,42 @@ struct GemmPtrs {
   const void *a_lo, *a_lo_sf, *a_hi, *a_hi_sf, *b_lo, *b_lo_sf, *b_hi, *b_hi_sf;
 };
 
-template <int BN, int CG>
+template <int BN, int CG, bool GATED = false>
 static int launch_gemm(const GemmPtrs& p, GemmArgs& g, cudaStream_t stream) {
   using C = GemmCfg<BN, CG>;
+  const int64_t b_rows = GATED ? 2 * static_cast<int64_t>(g.n) : g.n;
+  constexpr int kBBox = GATED ? 128 : C::kBRows, kSfBox = GATED ? 1 : C::kSfGroups;
   GemmMaps tm;
   memset(&tm, 0, sizeof(tm));
-  const int64_t mg = (g.m + 127) / 128, ng = (g.n + 127) / 128;
+  const int64_t mg = (g.m + 127) / 128, ng = (b_rows + 127) / 128;
   int st;
   if (g.k_lo) {
     if ((st = make_tmap(&tm.a_lo, p.a_lo, g.m, g.k_lo / 2, kBM)) != PLQ_OK) return st;
-    if ((st = make_tmap(&tm.b_lo, p.b_lo, g.n, g.k_lo / 2, C::kBRows)) != PLQ_OK) return st;
-    if (CG == 2 && (st = make_tmap(&tm.b_lo_half, p.b_lo, g.n, g.k_lo / 2, C::kBRows / 2)) != PLQ_OK) return st;
+    if ((st = make_tmap(&tm.b_lo, p.b_lo, b_rows, g.k_lo / 2, kBBox)) != PLQ_OK) return st;
+    if (CG == 2 && !GATED && (st = make_tmap(&tm.b_lo_half, p.b_lo, g.n, g.k_lo / 2, C::kBRows / 2)) != PLQ_OK) return st;
     if ((st = make_sf_tmap(&tm.sfa_lo, p.a_lo_sf, g.lo_chunks, mg, 1)) != PLQ_OK) return st;
-    if ((st = make_sf_tmap(&tm.sfb_lo, p.b_lo_sf, g.lo_chunks, ng, C::kSfGroups)) != PLQ_OK) return st;
+    if ((st = make_sf_tmap(&tm.sfb_lo, p.b_lo_sf, g.lo_chunks, ng, kSfBox)) != PLQ_OK) return st;
   }
   if (g.k_hi) {
     if ((st = make_tmap(&tm.a_hi, p.a_hi, g.m, g.k_hi, kBM)) != PLQ_OK) return st;
-    if ((st = make_tmap(&tm.b_hi, p.b_hi, g.n, g.k_hi, C::kBRows)) != PLQ_OK) return st;
-    if (CG == 2 && (st = make_tmap(&tm.b_hi_half, p.b_hi, g.n, g.k_hi, C::kBRows / 2)) != PLQ_OK) return st;
+    if ((st = make_tmap(&tm.b_hi, p.b_hi, b_rows, g.k_hi, kBBox)) != PLQ_OK) return st;
+    if (CG == 2 && !GATED && (st = make_tmap(&tm.b_hi_half, p.b_hi, g.n, g.k_hi, C::kBRows / 2)) != PLQ_OK) return st;
     if ((st = make_sf_tmap(&tm.sfa_hi, p.a_hi_sf, g.hi_chunks, mg, 1)) != PLQ_OK) return st;
-    if ((st = make_sf_tmap(&tm.sfb_hi, p.b_hi_sf, g.hi_chunks, ng, C::kSfGroups)) != PLQ_OK) return st;
+    if ((st = make_sf_tmap(&tm.sfb_hi, p.b_hi_sf, g.hi_chunks, ng, kSfBox)) != PLQ_OK) return st;
   }
   g.tiles_m = (g.m + kBM * CG - 1) / (kBM * CG);
-  g.tiles_n = (g.n + BN - 1) / BN;
+  g.tiles_n = static_cast<int>((b_rows + BN - 1) / BN);
   {
     // The operand that is walked in the inner direction is re-read once per step of the outer one and should
     // stay in L2.  M fastest (one band) re-reads A; when A is the larger operand and too big for that
     // (prefill down projection: 59 MB of A against 29 MB of B), narrow bands re-read B instead
     // (measured: 203 -> 187 us on that shape; 405 -> 446 us on gate_up, where B is the large one).
     const int64_t k_bytes = g.k_lo / 2 + g.k_hi;
-    const int64_t a_bytes = static_cast<int64_t>(g.m) * k_bytes, b_bytes = static_cast<int64_t>(g.n) * k_bytes;
+    const int64_t a_bytes = static_cast<int64_t>(g.m) * k_bytes, b_bytes = b_rows * k_bytes;
     g.band = (a_bytes > b_bytes && a_bytes > (32ll << 20)) ? 4 : g.tiles_m;
     if (g.band > g.tiles_m) g.band = g.tiles_m;
   }
-  auto kernel = mixed_gemm_kernel<BN, CG>;
+  auto kernel = mixed_gemm_kernel<BN, CG, GATED>;
   static thread_local int attr_dev = -1;
   int dev = 0;
   PLQ_CUDA_TRY(cudaGetDevice(&dev));
@@ -480,7 +516,7 @@ static int launch_gemm(const GemmPtrs& p, GemmArgs& g, cudaStream_t stream) {
   const int slots = sm_count() / CG;                 // CTAs (CG = 1) or CTA pairs (CG = 2) resident at once
   // The last wave is halved where twice its tiles still fit one wave.
   const int rest = tiles % slots;
-  g.full_tiles = CG == 2 && 2 * rest <= slots ? tiles - rest : tiles;
+  g.full_tiles = CG == 2 && !GATED && 2 * rest <= slots ? tiles - rest : tiles;
   const int items = 2 * tiles - g.full_tiles;
   const int groups = items < slots ? items : slots;
   cudaLaunchConfig_t cfg = {};
@@ -505,36 +541,46 @@ static int launch_gemm(const GemmPtrs& p, GemmArgs& g, cudaStream_t stream) {
 
 }  // namespace plq
 
+namespace plq {
+// Checks the arguments of a product and fills in what does not depend on the tile shape; `n` output columns, B has b_rows.
+static int gemm_setup(const GemmPtrs& p, int64_t m, int64_t n, int64_t b_rows, int64_t k_lo, int64_t k_hi, void* y_bf16, int64_t ldy,
+                      int32_t* dev_status, GemmArgs* g) {
+  if (m < 1 || n < 1 || k_lo < 0 || k_hi < 0 || k_lo + k_hi <= 0) return PLQ_ERR_SHAPE;
+  if (k_lo % 64 != 0 || k_hi % 32 != 0 || n % 8 != 0 || ldy % 8 != 0 || ldy < n) return PLQ_ERR_SHAPE;
+  if (m > (1 << 30) || b_rows > (1 << 30) || k_lo > (1 << 24) || k_hi > (1 << 24)) return PLQ_ERR_LIMIT;
+  if (!y_bf16 || !dev_status) return PLQ_ERR_NULL;
+  if (k_lo && (!p.a_lo || !p.a_lo_sf || !p.b_lo || !p.b_lo_sf)) return PLQ_ERR_NULL;
+  if (k_hi && (!p.a_hi || !p.a_hi_sf || !p.b_hi || !p.b_hi_sf)) return PLQ_ERR_NULL;
+  if (!aligned16(p.a_lo) || !aligned16(p.a_lo_sf) || !aligned16(p.a_hi) || !aligned16(p.a_hi_sf) || !aligned16(p.b_lo) ||
+      !aligned16(p.b_lo_sf) || !aligned16(p.b_hi) || !aligned16(p.b_hi_sf) || !aligned16(y_bf16))
+    return PLQ_ERR_ALIGN;
+  const int st = device_check();
+  if (st != PLQ_OK) return st;
+  g->y = static_cast<__nv_bfloat16*>(y_bf16);
+  g->ldy = ldy;
+  g->status = dev_status;
+  g->m = static_cast<int>(m); g->n = static_cast<int>(n);
+  g->up_row = static_cast<int>(n);
+  g->k_lo = static_cast<int>(k_lo); g->k_hi = static_cast<int>(k_hi);
+  g->lo_chunks = static_cast<int>(k_lo / 64);
+  g->hi_chunks = static_cast<int>((k_hi + 127) / 128);
+  g->lo_stages = (g->lo_chunks + 3) / 4;
+  g->hi_stages = g->hi_chunks;
+  g->wide_store = (reinterpret_cast<uintptr_t>(y_bf16) % 32 == 0 && ldy % 16 == 0) ? 1 : 0;
+  return PLQ_OK;
+}
+}  // namespace plq
+
 extern "C" int plq_mixed_gemm_variant(const void* a_lo_codes, const void* a_lo_sf, const void* a_hi_codes,
                                    const void* a_hi_sf, const void* b_lo_codes, const void* b_lo_sf,
                                    const void* b_hi_codes, const void* b_hi_sf, int64_t m, int64_t n, int64_t k_lo,
                                    int64_t k_hi, void* y_bf16, int64_t ldy, int32_t* dev_status, void* stream,
                                    int variant) {
   using namespace plq;
-  if (m < 1 || n < 1 || k_lo < 0 || k_hi < 0 || k_lo + k_hi <= 0) return PLQ_ERR_SHAPE;
-  if (k_lo % 64 != 0 || k_hi % 32 != 0 || n % 8 != 0 || ldy % 8 != 0 || ldy < n) return PLQ_ERR_SHAPE;
-  if (m > (1 << 30) || n > (1 << 30) || k_lo > (1 << 24) || k_hi > (1 << 24)) return PLQ_ERR_LIMIT;
-  if (!y_bf16 || !dev_status) return PLQ_ERR_NULL;
-  if (k_lo && (!a_lo_codes || !a_lo_sf || !b_lo_codes || !b_lo_sf)) return PLQ_ERR_NULL;
-  if (k_hi && (!a_hi_codes || !a_hi_sf || !b_hi_codes || !b_hi_sf)) return PLQ_ERR_NULL;
-  if (!aligned16(a_lo_codes) || !aligned16(a_lo_sf) || !aligned16(a_hi_codes) || !aligned16(a_hi_sf) ||
-      !aligned16(b_lo_codes) || !aligned16(b_lo_sf) || !aligned16(b_hi_codes) || !aligned16(b_hi_sf) ||
-      !aligned16(y_bf16))
-    return PLQ_ERR_ALIGN;
-  int st = device_check();
-  if (st != PLQ_OK) return st;
   GemmArgs g;
   const GemmPtrs ptrs = {a_lo_codes, a_lo_sf, a_hi_codes, a_hi_sf, b_lo_codes, b_lo_sf, b_hi_codes, b_hi_sf};
-  g.y = static_cast<__nv_bfloat16*>(y_bf16);
-  g.ldy = ldy;
-  g.status = dev_status;
-  g.m = static_cast<int>(m); g.n = static_cast<int>(n);
-  g.k_lo = static_cast<int>(k_lo); g.k_hi = static_cast<int>(k_hi);
-  g.lo_chunks = static_cast<int>(k_lo / 64);
-  g.hi_chunks = static_cast<int>((k_hi + 127) / 128);
-  g.lo_stages = (g.lo_chunks + 3) / 4;
-  g.hi_stages = g.hi_chunks;
-  g.wide_store = (reinterpret_cast<uintptr_t>(y_bf16) % 32 == 0 && ldy % 16 == 0) ? 1 : 0;
+  const int st = gemm_setup(ptrs, m, n, n, k_lo, k_hi, y_bf16, ldy, dev_status, &g);
+  if (st != PLQ_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (variant == PLQ_GEMM_AUTO) {
     // The cheapest shape is the one with the smallest (waves over the SMs) x (time of a whole wave); ties go to the larger
@@ -568,4 +614,21 @@ extern "C" int plq_mixed_gemm(const void* a_lo_codes, const void* a_lo_sf, const
                               int32_t* dev_status, void* stream) {
   return plq_mixed_gemm_variant(a_lo_codes, a_lo_sf, a_hi_codes, a_hi_sf, b_lo_codes, b_lo_sf, b_hi_codes, b_hi_sf,
                                 m, n, k_lo, k_hi, y_bf16, ldy, dev_status, stream, PLQ_GEMM_AUTO);
+}
+
+extern "C" int plq_mixed_gemm_silu_mul(const void* a_lo_codes, const void* a_lo_sf, const void* a_hi_codes, const void* a_hi_sf,
+                                       const void* b_lo_codes, const void* b_lo_sf, const void* b_hi_codes, const void* b_hi_sf,
+                                       int64_t m, int64_t n, int64_t k_lo, int64_t k_hi, void* y_bf16, int64_t ldy,
+                                       int32_t* dev_status, void* stream) {
+  using namespace plq;
+  if (n % 128 != 0) return PLQ_ERR_SHAPE;            // the up rows start on a 128-row group of scales
+  GemmArgs g;
+  const GemmPtrs ptrs = {a_lo_codes, a_lo_sf, a_hi_codes, a_hi_sf, b_lo_codes, b_lo_sf, b_hi_codes, b_hi_sf};
+  const int st = gemm_setup(ptrs, m, n, 2 * n, k_lo, k_hi, y_bf16, ldy, dev_status, &g);
+  if (st != PLQ_OK) return st;
+  // waves times the time of a wave, as in plq_mixed_gemm_variant
+  const int64_t sms = sm_count(), slots = sms / 2 > 0 ? sms / 2 : 1;
+  const int64_t pair = ((m + 255) / 256 * (n / 128) + slots - 1) / slots * 100, wide = ((m + 127) / 128 * (n / 128) + sms - 1) / sms * 120;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  return wide < pair ? launch_gemm<256, 1, true>(ptrs, g, s) : launch_gemm<256, 2, true>(ptrs, g, s);
 }

@@ -26,6 +26,7 @@ struct Api {
   decltype(&::plq_silu_mul_pack) silu_mul_pack;
   decltype(&::plq_gemv_tc) gemv_tc;
   decltype(&::plq_mixed_gemm) mixed_gemm;
+  decltype(&::plq_mixed_gemm_silu_mul) mixed_gemm_silu_mul;
   decltype(&::plq_rope_kv_append) rope_kv_append;
   decltype(&::plq_rope_kv_append_nvfp4_values) rope_kv_append_nvfp4_values;
   decltype(&::plq_sf_tiled_bytes) sf_tiled_bytes;
@@ -45,6 +46,7 @@ void init(const std::string& path) {
   find(api.silu_mul_pack, "plq_silu_mul_pack");
   find(api.gemv_tc, "plq_gemv_tc");
   find(api.mixed_gemm, "plq_mixed_gemm");
+  find(api.mixed_gemm_silu_mul, "plq_mixed_gemm_silu_mul");
   find(api.rope_kv_append, "plq_rope_kv_append");
   find(api.rope_kv_append_nvfp4_values, "plq_rope_kv_append_nvfp4_values");
   find(api.sf_tiled_bytes, "plq_sf_tiled_bytes");
@@ -231,6 +233,7 @@ std::tuple<Tensor, Tensor> decoder_layer(const Linear& qkv, const Linear& o, con
   const int64_t out_rows = last_only ? b : rows;
   Tensor h2 = at::empty_like(h1), delta2 = at::empty_like(h1);
   uint8_t* gu = act + out0;
+  const bool gated = like > 16 && ffn % 128 == 0;      // the GEMM applies SiLU(gate) * up itself
   {
     const PackedAt p(ws.data_ptr(), out_rows, o.k_lo, o.k_hi);
     check(api.pack(attn.const_data_ptr(), out_rows, attn_width, o.k_hi, 1, p.lo, p.lo_sf, p.hi, p.hi_sf, PLQ_SF_TILED, stream));
@@ -240,11 +243,18 @@ std::tuple<Tensor, Tensor> decoder_layer(const Linear& qkv, const Linear& o, con
     const PackedAt p(ws.data_ptr(), out_rows, gate_up.k_lo, gate_up.k_hi);
     check(api.add_rmsnorm_pack(act, h1.const_data_ptr(), h2.data_ptr(), ln2.const_data_ptr(), eps, out_rows, hidden, gate_up.k_hi, 1, p.lo,
                                p.lo_sf, p.hi, p.hi_sf, PLQ_SF_TILED, stream));
-    check(gate_up.product(p, out_rows, gu, 2 * ffn, stream, like));
+    if (gated)
+      check(api.mixed_gemm_silu_mul(p.lo, p.lo_sf, p.hi, p.hi_sf, ptr(gate_up.lo), ptr(gate_up.lo_sf), ptr(gate_up.hi), ptr(gate_up.hi_sf),
+                                    out_rows, ffn, gate_up.k_lo, gate_up.k_hi, gu, ffn, status, stream));
+    else
+      check(gate_up.product(p, out_rows, gu, 2 * ffn, stream, like));
   }
   {
     const PackedAt p(ws.data_ptr(), out_rows, down.k_lo, down.k_hi);
-    check(api.silu_mul_pack(gu, gu + 2 * ffn, 2 * ffn, out_rows, ffn, down.k_hi, 1, p.lo, p.lo_sf, p.hi, p.hi_sf, PLQ_SF_TILED, stream));
+    if (gated)
+      check(api.pack(gu, out_rows, ffn, down.k_hi, 1, p.lo, p.lo_sf, p.hi, p.hi_sf, PLQ_SF_TILED, stream));
+    else
+      check(api.silu_mul_pack(gu, gu + 2 * ffn, 2 * ffn, out_rows, ffn, down.k_hi, 1, p.lo, p.lo_sf, p.hi, p.hi_sf, PLQ_SF_TILED, stream));
     check(down.product(p, out_rows, delta2.data_ptr(), hidden, stream, like));
   }
   return {h2, delta2};

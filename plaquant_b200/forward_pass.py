@@ -366,6 +366,14 @@ class ResQForwardB200:
         self._kv_room[li] = (weakref.ref(k), weakref.ref(v), cap)
         return k, v, n, cap
 
+    def _gate_up(self, L: _Layer, pa: ops.PackedMatrix, like: int) -> ops.PackedMatrix:
+        """down_proj's packed input: gate_up, SiLU(gate) * up, rotation, quantisation.  Batches on the GEMM (more than 16
+        rows in the whole pass) get the activation from the product's own epilogue."""
+        if like > 16 and type(L.gate_up) is QuantizedLinear and self.ffn % 128 == 0 and L.gate_up._gemm_w is not None:
+            return ops.pack(ops.mixed_gemm_silu_mul(pa, L.gate_up._gemm_w), self.k_hi_ffn, hadamard=True)
+        gu = L.gate_up(pa)                                                              # [rows, 2 * ffn] = [gate | up]
+        return ops.silu_mul_pack(gu, self.k_hi_ffn)
+
     def _plain_layer(self, L: _Layer) -> bool:
         """Is the layer made of this package's plain linears and norm weights (what the native call takes)?"""
         for lin in (L.qkv, L.o, L.gate_up, L.down):
@@ -429,7 +437,7 @@ class ResQForwardB200:
             h = h[:, -1:].contiguous()
             o = ops.mixed_gemm(L.o.quantize_input(attn[:, -1]), L.o._gemm_w).view(h.shape)
             h, pa = ops.add_rmsnorm_pack(o, h, L.ln2, c.rms_eps, self.k_hi_hidden)
-            pa = ops.silu_mul_pack(ops.mixed_gemm(pa, L.gate_up._gemm_w), self.k_hi_ffn)
+            pa = self._gate_up(L, pa, like=b * t)
             return h, ops.mixed_gemm(pa, L.down._gemm_w).view(h.shape)
         if fused:
             L.o(attn.reshape(b * t, -1), out=self.peer.buffer(b * t))                   # partial sums stay in the peer buffer
@@ -437,8 +445,7 @@ class ResQForwardB200:
         else:
             o = self.ctx.all_reduce(self._quantized_linear(attn, L.o))
             h, pa = ops.add_rmsnorm_pack(o, h, L.ln2, c.rms_eps, self.k_hi_hidden)      # h += o; RMSNorm(ln2); quantise
-        gu = L.gate_up(pa)                                                              # [b*t, 2*ffn] = [gate | up]
-        pa = ops.silu_mul_pack(gu, self.k_hi_ffn)                                       # SiLU(gate)*up; rotate; quantise
+        pa = self._gate_up(L, pa, like=b * t)
         if fused:
             L.down(pa, out=self.peer.buffer(b * t))       # reduced by the next layer's first kernel (or _finish)
             return h, _IN_PEER_BUFFER
@@ -497,7 +504,7 @@ class ResQForwardB200:
             attn = self._attention(li, L.qkv(pa).view(b, t, -1), 0, cos_sin, None)
             L.o(attn.reshape(R, -1), out=sr.buffer(R))
             h, pa = ops.reduce_scatter_add_rmsnorm_pack(sr, R, h, L.ln2, c.rms_eps)
-            pa = ops.silu_mul_pack(L.gate_up(pa), self.k_hi_ffn)
+            pa = self._gate_up(L, pa, like=R)
             L.down(pa, out=sr.buffer(R))
         h, _ = ops.reduce_scatter_add_rmsnorm_pack(sr, R, h, self.final_norm, c.rms_eps)     # last add; packed rows unused
         self.pos = t

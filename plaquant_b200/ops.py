@@ -331,6 +331,20 @@ def mixed_gemm(a: PackedMatrix, b: PackedMatrix, out: Optional[torch.Tensor] = N
     return y
 
 
+def mixed_gemm_silu_mul(a: PackedMatrix, b: PackedMatrix) -> torch.Tensor:
+    """SiLU(gate) * up of [gate | up] = deq(a) @ deq(b).T, bf16 [m, b.rows / 2]; b.rows a multiple of 256.  The same values
+    as mixed_gemm and the SiLU prologue of silu_mul_pack behind it."""
+    _check_pair(a, b, SF_TILED)
+    n = b.rows // 2
+    y = torch.empty(a.rows, n, dtype=torch.bfloat16, device=a.device)
+    with torch.cuda.device(a.device):
+        st = _lib.lib().plq_mixed_gemm_silu_mul(
+            _ptr(a.lo_codes), _ptr(a.lo_sf), _ptr(a.hi_codes), _ptr(a.hi_sf), _ptr(b.lo_codes), _ptr(b.lo_sf), _ptr(b.hi_codes),
+            _ptr(b.hi_sf), a.rows, n, a.k_lo, a.k_hi, _ptr(y), n, _ptr(status_word(a.device)), _stream(a.device))
+    _lib.check(st)
+    return y
+
+
 _gemv_ws = {}
 
 

@@ -195,3 +195,22 @@ def test_half_tiles_of_the_last_wave_equal_other_tile_shapes(m, n, k, k_hi):
     assert np.array_equal(y, _run(pa, pb, None))
     if n < 1000:
         assert rel_l2(y, _oracle_bf16(packed_to_numpy(pa), packed_to_numpy(pb))) <= TOL
+
+
+# m: one row, past a CTA, past a pair, several row tiles, one wave and more; n: one tile and several; k: ragged last stages
+# of both formats, one format only, more stages than the ring
+@pytest.mark.parametrize("m,n,k,k_hi", [(1, 128, 128, 64), (17, 256, 1024, 64), (129, 128, 192, 64), (300, 384, 384, 384),
+                                        (333, 512, 14336, 448), (1000, 256, 448, 0), (77, 14336, 512, 64), (600, 9728, 256, 64)])
+def test_silu_mul_in_the_epilogue_equals_gemm_and_silu_prologue(m, n, k, k_hi):
+    x, w = synth_activation(m, k, seed=m + k).cuda(), synth_weight(2 * n, k, seed=n + k).cuda() * 4
+    x[0, :2] = 1e4                                                     # some gates far out on both sides
+    had = k % 128 == 0
+    pa, pb = (plq.pack(t, k_hi, hadamard=had, sf_layout="tiled") for t in (x, w))
+    from plaquant_b200 import ops
+    got = ops.mixed_gemm_silu_mul(pa, pb)
+    plq.check_device_status()
+    gu = f32_of(plq.mixed_gemm(pa, pb))
+    want = F.silu_mul_bf16(gu[:, :n], gu[:, n:])
+    assert np.array_equal(f32_of(got), want)
+    with pytest.raises(plq.PlqError):                                  # up rows inside a 128-row group of scales
+        ops.mixed_gemm_silu_mul(pa, plq.pack(w[:208], k_hi, hadamard=had, sf_layout="tiled"))
