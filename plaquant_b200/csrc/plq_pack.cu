@@ -34,6 +34,10 @@ namespace plq {
 #define PLQ_PACK_TARGET_THREADS 128
 #endif
 constexpr int kPackTargetThreads = PLQ_PACK_TARGET_THREADS;   // CTA size the launcher aims for (whole rows)
+// Rotated rows go to pack_rows_kernel up to this many of its warps per SM
+#ifndef PLQ_PACK_ROWS_WARPS
+#define PLQ_PACK_ROWS_WARPS 16
+#endif
 
 struct PackArgs {
   const uint4* x;        // bf16 [rows, k], row stride ldx8 * 8 elements
@@ -149,6 +153,20 @@ __device__ __forceinline__ void store_run_nvfp4(const PackArgs& a, const uint4& 
   store_out<PRO>(a, 0, a.lo_codes, (static_cast<size_t>(row) * a.k_lo + o) / 2, codes);
 }
 
+// The scale byte of the MXFP8 block that starts at column k_lo + kh.
+template <int PRO>
+__device__ __forceinline__ void store_scale_mxfp8(const PackArgs& a, uint32_t c, int row, int kh) {
+  const int k_hi = a.k - a.k_lo, kb = kh >> 5;
+  const size_t off = a.sf_tiled ? static_cast<size_t>(sf_tiled_offset(row, kb, a.hi_chunks))
+                                : static_cast<size_t>(row) * (k_hi >> 5) + kb;
+  store_out<PRO>(a, 3, a.hi_sf, off, static_cast<uint8_t>(c));
+  // The row's last block also writes the zero scales up to the end of its chunk: a buffer cleared beforehand would be
+  // one more launch per call (K = 14336: 14 scales in 16).
+  if (a.sf_tiled && kb + 1 == (k_hi >> 5))
+    for (int z = kb + 1; z < 4 * a.hi_chunks; ++z)
+      store_out<PRO>(a, 3, a.hi_sf, static_cast<size_t>(sf_tiled_offset(row, z, a.hi_chunks)), static_cast<uint8_t>(0));
+}
+
 // The same for a run in the MXFP8 columns (o >= k_lo): 32 code bytes and one scale byte.
 template <int PRO>
 __device__ __forceinline__ void quantize_run_mxfp8(const PackArgs& a, const float2* v, int row, int o) {
@@ -160,15 +178,7 @@ __device__ __forceinline__ void quantize_run_mxfp8(const PackArgs& a, const floa
   const size_t coff = static_cast<size_t>(row) * k_hi + kh;
   store_out<PRO>(a, 2, a.hi_codes, coff, make_uint4(c0.x, c0.y, c1.x, c1.y));
   store_out<PRO>(a, 2, a.hi_codes, coff + 16, make_uint4(c2.x, c2.y, c3.x, c3.y));
-  const int kb = kh >> 5;
-  const size_t off = a.sf_tiled ? static_cast<size_t>(sf_tiled_offset(row, kb, a.hi_chunks))
-                                : static_cast<size_t>(row) * (k_hi >> 5) + kb;
-  store_out<PRO>(a, 3, a.hi_sf, off, static_cast<uint8_t>(c));
-  // The row's last block also writes the zero scales up to the end of its chunk: a buffer cleared beforehand would be
-  // one more launch per call (K = 14336: 14 scales in 16).
-  if (a.sf_tiled && kb + 1 == (k_hi >> 5))
-    for (int z = kb + 1; z < 4 * a.hi_chunks; ++z)
-      store_out<PRO>(a, 3, a.hi_sf, static_cast<size_t>(sf_tiled_offset(row, z, a.hi_chunks)), static_cast<uint8_t>(0));
+  store_scale_mxfp8<PRO>(a, c, row, kh);
 }
 
 // ---- staging through shared memory -------------------------------------------------------
@@ -652,6 +662,158 @@ __global__ void PLQ_PACK_BOUNDS pack_kernel(const PackArgs a) {
   }
 }
 
+// ---- the same for a few rows ------------------------------------------------------------------------------------------
+// A decode batch leaves the kernel above with one warp per scheduler, and what it takes is the length of that warp's
+// chain: ~950 instructions over 64 elements per lane.  Here a lane has 16 elements (one NVFP4 block, an eighth of a
+// rotation block), a warp 512, loaded straight into registers: a quarter of the chain, three more exchanges between lanes
+// per element (strides 16, 32, 64).  Rotated rows only; the same operations in the same order, bit for bit:
+//   * sum of squares: a 32-element run is two lanes, the second continues the first's chains; chunks of 64 meet in the
+//     same pairwise tree, its last two levels through shared memory;
+//   * butterflies: v +- partner is one fused multiply-add with a factor of +-1, rounded once.
+template <int PRO, bool NORM>
+__global__ void __launch_bounds__(NORM ? 1024 : 128) pack_rows_kernel(const PackArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int wpr = (a.k + 511) >> 9;                 // warps (512-element segments) per row
+  int row = blockIdx.x, seg = warp;                 // with a norm a CTA is a row
+  if constexpr (!NORM) {
+    const int u = static_cast<int>(blockIdx.x) * 4 + warp;
+    row = u / wpr;
+    seg = u - row * wpr;
+    if (row >= a.rows) return;
+  }
+  const int e0 = 512 * seg + 16 * lane;             // the lane's first element
+  const bool ok = e0 < a.k;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  const size_t r0 = static_cast<size_t>(row);
+  const uint4* px = a.x + r0 * a.ldx8 + (e0 >> 3);
+  const uint4 wx[2] = {ok ? px[0] : zero, ok ? px[1] : zero};
+  uint4 wy[2] = {zero, zero}, wg[2] = {zero, zero};
+  if constexpr (PRO != 0) {
+    const uint4* py = a.x2 + r0 * (PRO == 1 ? a.ldx8 : a.k >> 3) + (e0 >> 3);
+    if (ok) { wy[0] = py[0]; wy[1] = py[1]; }
+  }
+  if constexpr (NORM) {
+    if (ok) { wg[0] = a.gamma[e0 >> 3]; wg[1] = a.gamma[(e0 >> 3) + 1]; }
+  }
+  float2 v[8];                                      // elements (e0 + 2 i, e0 + 2 i + 1)
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const uint32_t x[4] = {wx[c].x, wx[c].y, wx[c].z, wx[c].w}, y[4] = {wy[c].x, wy[c].y, wy[c].z, wy[c].w};
+    uint32_t h[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float2& o = v[4 * c + i];
+      if constexpr (PRO == 0) {
+        o = enter_pair<!NORM>(x[i]);
+      } else if constexpr (PRO == 1) {
+        const float2 sl = silu2(make_float2(bf16lo_to_f32(x[i]), bf16hi_to_f32(x[i])));
+        const uint32_t t = f32x2_to_bf16x2(sl.x, sl.y);
+        const float2 prod = __fmul2_rn(make_float2(bf16lo_to_f32(t), bf16hi_to_f32(t)), make_float2(bf16lo_to_f32(y[i]), bf16hi_to_f32(y[i])));
+        o = enter_pair<true>(f32x2_to_bf16x2(prod.x, prod.y));
+      } else {
+        const float2 sum = __fadd2_rn(make_float2(bf16lo_to_f32(y[i]), bf16hi_to_f32(y[i])), make_float2(bf16lo_to_f32(x[i]), bf16hi_to_f32(x[i])));
+        h[i] = f32x2_to_bf16x2(sum.x, sum.y);
+        o = make_float2(bf16lo_to_f32(h[i]), bf16hi_to_f32(h[i]));
+      }
+    }
+    if constexpr (PRO == 2)
+      if (ok) a.h_out[r0 * (a.k >> 3) + (e0 >> 3) + c] = make_uint4(h[0], h[1], h[2], h[3]);
+  }
+
+  if constexpr (NORM) {
+    __shared__ float sums[32];
+    float2 s = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s = __ffma2_rn(v[i], v[i], s);
+    s.x = __shfl_xor_sync(0xFFFFFFFFu, s.x, 1);
+    s.y = __shfl_xor_sync(0xFFFFFFFFu, s.y, 1);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s = __ffma2_rn(v[i], v[i], s);       // odd lanes: the run's chains; even lanes: unused
+    float t = __fadd_rn(s.x, s.y);
+    t = t + __shfl_xor_sync(0xFFFFFFFFu, t, 2);                      // the two runs of a 64-element chunk
+    t = t + __shfl_xor_sync(0xFFFFFFFFu, t, 4);
+    t = t + __shfl_xor_sync(0xFFFFFFFFu, t, 8);
+    t = t + __shfl_xor_sync(0xFFFFFFFFu, t, 16);
+    if (lane == 1) sums[warp] = t;
+    const int padded = (wpr + 3) & ~3;
+    if (threadIdx.x < padded - wpr) sums[wpr + threadIdx.x] = 0.0f;
+    __syncthreads();
+    float tot = 0.0f;
+    for (int w = 0; w < padded; w += 4) tot = tot + ((sums[w] + sums[w + 1]) + (sums[w + 2] + sums[w + 3]));
+    const float var = __fdiv_rn(tot, static_cast<float>(a.k));
+    const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(var, a.eps)));
+    const float2 r2 = make_float2(r, r);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      float2 g[4];
+      unpack8(wg[c], g);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 y = __fmul2_rn(g[i], __fmul2_rn(v[4 * c + i], r2));
+        v[4 * c + i] = enter_pair<true>(f32x2_to_bf16x2(y.x, y.y));
+      }
+    }
+  }
+
+  const float2 neg1 = make_float2(-1.0f, -1.0f);
+#pragma unroll
+  for (int h = 1; h < 8; h <<= 1) {                  // strides 2, 4, 8 (stride 1: enter_pair)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if ((i & h) == 0) {
+        const float2 x0 = v[i], x1 = v[i + h];
+        v[i] = __fadd2_rn(x0, x1);
+        v[i + h] = __ffma2_rn(x1, neg1, x0);
+      }
+    }
+  }
+#pragma unroll
+  for (int h = 1; h < 8; h <<= 1) {                  // strides 16, 32, 64: the upper lane holds partner - own
+    const float sg = (lane & h) ? -1.0f : 1.0f;
+    const float2 sg2 = make_float2(sg, sg);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float2 o;
+      o.x = __shfl_xor_sync(0xFFFFFFFFu, v[i].x, h);
+      o.y = __shfl_xor_sync(0xFFFFFFFFu, v[i].y, h);
+      v[i] = __ffma2_rn(v[i], sg2, o);
+    }
+  }
+  const float c128 = 0.088388347648318441f;          // 1/sqrt(128), then to bf16
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = round_bf16_pair(__fmul2_rn(v[i], make_float2(c128, c128)));
+
+  const float m = absmax<8>(v);
+  const bool hi = e0 >= a.k_lo;
+  const uint32_t c = nvfp4_scale_code(m);
+  const float rs = rcp_approx(e4m3_code_to_f32(c));
+  const uint2 codes = make_uint2(nvfp4_quantize8(v, rs), nvfp4_quantize8(v + 4, rs));
+  uint32_t sf = c << (8 * (lane & 3));               // four blocks' scales to one word
+  sf |= __shfl_xor_sync(0xFFFFFFFFu, sf, 1);
+  sf |= __shfl_xor_sync(0xFFFFFFFFu, sf, 2);
+  if (ok && !hi) {
+    *reinterpret_cast<uint2*>(a.lo_codes + (r0 * a.k_lo + e0) / 2) = codes;
+    if ((lane & 3) == 0) {
+      const int kb = e0 >> 4;
+      const size_t off = a.sf_tiled ? static_cast<size_t>(sf_tiled_offset(row, kb, a.lo_chunks)) : r0 * (a.k_lo >> 4) + kb;
+      *reinterpret_cast<uint32_t*>(a.lo_sf + off) = sf;
+    }
+  }
+  if (__any_sync(0xFFFFFFFFu, ok && hi)) {           // MXFP8 columns: a block is two lanes
+    const float m2 = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, 1));
+    const uint32_t c8 = mxfp8_scale_code(m2);
+    const float inv = __uint_as_float((254u - c8) << 23);
+    const uint2 q0 = mxfp8_quantize8(v, inv), q1 = mxfp8_quantize8(v + 4, inv);
+    if (ok && hi) {
+      const int k_hi = a.k - a.k_lo, kh = e0 - a.k_lo;
+      *reinterpret_cast<uint4*>(a.hi_codes + r0 * k_hi + kh) = make_uint4(q0.x, q0.y, q1.x, q1.y);
+      if ((lane & 1) == 0) store_scale_mxfp8<0>(a, c8, row, kh);
+    }
+  }
+}
+
 // ---- dequantise packed -> bf16 [rows, k]; one thread per 8 elements -------------------------
 struct UnpackArgs {
   const uint8_t *lo_codes, *lo_sf, *hi_codes, *hi_sf;
@@ -800,6 +962,25 @@ static int launch_pack(int pro, const void* x, const void* x2, void* h_out, int6
   a.sf_tiled = sf_layout == PLQ_SF_TILED;
   a.lo_chunks = static_cast<int>(((k - k_hi) / 16 + 3) / 4);
   a.hi_chunks = static_cast<int>((k_hi / 32 + 3) / 4);
+  const int64_t small_wpr = (k + 511) / 512;
+  if (hadamard && pro != 3 && rows * small_wpr <= PLQ_PACK_ROWS_WARPS * static_cast<int64_t>(sm_count()) && (!norm || small_wpr <= 32)) {
+    auto launch_rows = [&](void (*kernel)(const PackArgs)) -> int {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(static_cast<unsigned>(norm ? rows : (rows * small_wpr + 3) / 4), 1, 1);
+      cfg.blockDim = dim3(static_cast<unsigned>(norm ? 32 * small_wpr : 128), 1, 1);
+      cfg.stream = static_cast<cudaStream_t>(stream);
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[0].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      PLQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, a));
+      return PLQ_OK;
+    };
+    if (pro == 1) return norm ? PLQ_ERR_SHAPE : launch_rows(pack_rows_kernel<1, false>);
+    if (pro == 2) return norm ? launch_rows(pack_rows_kernel<2, true>) : PLQ_ERR_NULL;
+    return norm ? launch_rows(pack_rows_kernel<0, true>) : launch_rows(pack_rows_kernel<0, false>);
+  }
   // threads per row: one per 64 elements, whole warps.  With a row norm a CTA holds whole rows: as many as fit the
   // target CTA size, fewer when the groups would not cover the GPU a few times over (decode batches).  Without one
   // the unit of work is a row segment (one warp) and a CTA takes any `warps` of them.
