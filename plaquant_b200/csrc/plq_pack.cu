@@ -34,9 +34,11 @@ namespace plq {
 #define PLQ_PACK_TARGET_THREADS 128
 #endif
 constexpr int kPackTargetThreads = PLQ_PACK_TARGET_THREADS;   // CTA size the launcher aims for (whole rows)
-// Rotated rows go to pack_rows_kernel up to this many of its warps per SM
+// Rotated rows go to pack_rows_kernel up to this many of its warps per SM (one resident set).  Replayed, this kernel against
+// pack_kernel: m = 16, K = 4096 norm 2.40 / 3.97 us, residual + norm 2.61 / 4.50; 333 rows 4.0 / 5.2 and 4.9 / 6.4; 8192 x 512
+// (55 warps per SM) 7.3 / 7.1 and 9.2 / 12.2; K = 14336, 333 rows (63) plain 5.0 / 5.4, SiLU 6.8 / 9.3.
 #ifndef PLQ_PACK_ROWS_WARPS
-#define PLQ_PACK_ROWS_WARPS 16
+#define PLQ_PACK_ROWS_WARPS 64
 #endif
 
 struct PackArgs {
