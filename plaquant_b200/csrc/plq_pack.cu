@@ -34,12 +34,12 @@ namespace plq {
 #define PLQ_PACK_TARGET_THREADS 128
 #endif
 constexpr int kPackTargetThreads = PLQ_PACK_TARGET_THREADS;   // CTA size the launcher aims for (whole rows)
-// Rotated rows go to pack_rows_kernel up to this many of its warps per SM (one resident set).  Replayed, this kernel against
-// pack_kernel: m = 16, K = 4096 norm 2.40 / 3.97 us, residual + norm 2.61 / 4.50; 333 rows 4.0 / 5.2 and 4.9 / 6.4; 8192 x 512
-// (55 warps per SM) 7.3 / 7.1 and 9.2 / 12.2; K = 14336, 333 rows (63) plain 5.0 / 5.4, SiLU 6.8 / 9.3.
-#ifndef PLQ_PACK_ROWS_WARPS
-#define PLQ_PACK_ROWS_WARPS 64
-#endif
+// Rotated rows go to pack_rows_kernel up to this many of its warps per SM: one resident set (64) with a norm alone, whose
+// warps wait for each other; two where a residual is added or nothing is; four with SiLU.  Replayed, this kernel against
+// pack_kernel, us: m = 16, K = 4096 norm 2.4 / 4.0, residual + norm 2.6 / 4.5; m = 333 norm 4.0 / 5.2; 8192 x 512 (55 warps
+// per SM) norm 7.3 / 7.1; 4096 x 2048 (111) plain 7.7 / 8.8, SiLU 10.4 / 12.6, norm 10.7 / 10.6, residual + norm 13.7 / 15.0;
+// 4096 x 4096 (221) plain 13.9 / 13.4, SiLU 19.1 / 21.2, residual + norm 27.0 / 26.9.
+constexpr int pack_rows_warps(int pro, bool norm) { return pro == 1 ? 256 : norm && pro == 0 ? 64 : 128; }
 
 struct PackArgs {
   const uint4* x;        // bf16 [rows, k], row stride ldx8 * 8 elements
@@ -965,7 +965,7 @@ static int launch_pack(int pro, const void* x, const void* x2, void* h_out, int6
   a.lo_chunks = static_cast<int>(((k - k_hi) / 16 + 3) / 4);
   a.hi_chunks = static_cast<int>((k_hi / 32 + 3) / 4);
   const int64_t small_wpr = (k + 511) / 512;
-  if (hadamard && pro != 3 && rows * small_wpr <= PLQ_PACK_ROWS_WARPS * static_cast<int64_t>(sm_count()) && (!norm || small_wpr <= 32)) {
+  if (hadamard && pro != 3 && rows * small_wpr <= pack_rows_warps(pro, norm) * static_cast<int64_t>(sm_count()) && (!norm || small_wpr <= 32)) {
     auto launch_rows = [&](void (*kernel)(const PackArgs)) -> int {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(static_cast<unsigned>(norm ? rows : (rows * small_wpr + 3) / 4), 1, 1);

@@ -136,7 +136,7 @@ __device__ __forceinline__ uint2 mxfp8_quantize8(const float2* x, float inv) {
 __device__ __forceinline__ float e8m0_to_f32(uint32_t code) { return __uint_as_float(code << 23); }
 
 // ---- SiLU ------------------------------------------------------------------------------------
-// SiLU(g) = g / (1 + exp(-g)) of a bf16-valued g, to be rounded to bf16 by the caller.  The CPU checker defines it
+// SiLU(g) = g / (1 + exp(-g)) of a bf16-valued g, to be rounded to bf16 by the caller.  The CPU oracle defines it
 // with a float32 exponential written down operation by operation and an IEEE division (silu_mul_bf16 / exp_det); the
 // value needed is its rounding to 8 significant bits for one of 65 280 possible inputs, and the hardware's ex2 and
 // rcp approximations (a few units in the 24th bit) give the same bf16 for every one of them - the GPU tests compare
