@@ -146,7 +146,7 @@ struct Linear {
                                    p.lo_sf, p.hi, p.hi_sf, PLQ_SF_TILED, stream)
                 : api.pack(x2.const_data_ptr(), rows, k(), k_hi, hadamard, p.lo, p.lo_sf, p.hi, p.hi_sf, PLQ_SF_TILED, stream));
     check(product(p, rows, y.data_ptr(), y.stride(0), stream));
-    if (x.dim() == 2) return y;
+    if (x.dim() == 2 && !out) return y;
     std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
     shape.back() = n;
     return y.view(shape);

@@ -307,6 +307,17 @@ def _check_pair(a: PackedMatrix, b: PackedMatrix, layout: int) -> None:
         raise ValueError("scale buffers are in the wrong layout for this kernel")
 
 
+def check_out(out: torch.Tensor, rows: int, n: int, device) -> None:
+    """A caller's output buffer for [rows, n]: bf16 on `device`, `rows` rows of `n` neighbouring elements (the rows may be
+    further apart).  The kernels get its address and row stride alone, so what does not fit is refused before a launch."""
+    if out.dtype != torch.bfloat16:
+        raise TypeError("out must be bfloat16")
+    if out.device != device:
+        raise RuntimeError(f"out is on {out.device}, the product on {device}")
+    if out.dim() < 2 or out.shape[0] != rows or out.numel() != rows * n or (rows and not out[0].is_contiguous()):
+        raise RuntimeError(f"out {tuple(out.shape)} with strides {tuple(out.stride())} does not hold [{rows}, {n}] with contiguous rows")
+
+
 def native_linear(w: PackedMatrix):
     """The front end's object for a packed weight (tiled scales), complete before any call that uses it."""
     return _lib.torch_lib().Linear(w.lo_codes, w.lo_sf, w.hi_codes, w.hi_sf, status_word(w.device), w.rows, w.k_lo, w.k_hi)

@@ -123,11 +123,15 @@ class QuantizedLinear:
     def forward(self, x, norm_weight: Optional[torch.Tensor] = None, eps: float = 1e-6,
                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """x: bf16 [..., K] (or an already packed PackedMatrix).  `norm_weight` fuses the preceding
-        RMSNorm (inference/forward_pass.py:33-39) into the quantisation kernel."""
+        RMSNorm (inference/forward_pass.py:33-39) into the quantisation kernel.  `out`: bf16 [rows, N] to write to, its rows
+        contiguous; the result is a view of it."""
         if self.gemm_impl != "b200":
             raise ValueError(f"Unknown gemm_impl: {self.gemm_impl}")
         if self._gemm_w is None:
             raise RuntimeError("QuantizedLinear weights are not on a CUDA device; call .to('cuda') (no CPU path)")
+        if out is not None:
+            rows = x.rows if isinstance(x, ops.PackedMatrix) else x.shape[:-1].numel()
+            ops.check_out(out, rows, self.out_features, self._gemm_w.device)
         if isinstance(x, torch.Tensor):
             y = self.native().forward(x, self.online_had, norm_weight, eps, out)
             if y is not None:

@@ -77,3 +77,21 @@ def test_torch_front_end_loads_and_leaves_cpu_tensors_to_the_caller(lib):
     u8 = torch.zeros(0, dtype=torch.uint8)
     lin = fe.Linear(u8, u8, u8, u8, torch.zeros(1, dtype=torch.int32), 8, 192, 64)
     assert lin.forward(torch.zeros(1, 256, dtype=torch.bfloat16), False, None, 1e-6, None) is None
+
+
+def test_outputs_that_do_not_fit_are_refused():
+    """Only the address and the row stride of `out` reach a kernel: every form that would be written past its end, between
+    its elements or as another type is refused on the host."""
+    import torch
+    from plaquant_b200 import ops
+    cpu, bf = torch.device("cpu"), torch.bfloat16
+    for good in (torch.empty(5, 16, dtype=bf), torch.empty(5, 32, dtype=bf)[:, 8:24], torch.empty(5, 1, 16, dtype=bf), torch.empty(10, 16, dtype=bf)[::2]):
+        ops.check_out(good, 5, 16, cpu)
+    for bad in (torch.empty(5, 24, dtype=bf), torch.empty(4, 16, dtype=bf), torch.empty(6, 16, dtype=bf), torch.empty(80, dtype=bf),
+                torch.empty(16, 5, dtype=bf), torch.empty(16, 5, dtype=bf).t(), torch.empty(5, 32, dtype=bf)[:, ::2], torch.empty(1, 5, 16, dtype=bf),
+                torch.empty(5, 16, dtype=bf, device="meta")):
+        with pytest.raises(RuntimeError):
+            ops.check_out(bad, 5, 16, cpu)
+    for dtype in (torch.float16, torch.float32, torch.int16):
+        with pytest.raises(TypeError):
+            ops.check_out(torch.empty(5, 16, dtype=dtype), 5, 16, cpu)

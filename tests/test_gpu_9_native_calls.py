@@ -100,3 +100,28 @@ def test_last_position_logits_equal_those_of_every_position(monkeypatch, rows_li
     assert all(torch.equal(x[:, -1], y[:, -1]) for x, y in zip(whole, short))
     assert short[0].shape[1] == (1 if b * t > 16 else t)
     plq.check_device_status()
+
+
+@pytest.mark.parametrize("rows", [1, 16, 17])
+def test_linear_refuses_an_output_that_does_not_fit(rows):
+    """Every route to the product - a tensor, a packed operand in either layout - looks at `out` before it launches."""
+    from plaquant_b200 import ops
+    from plaquant_b200.quantize import QuantizedLinear
+    lin = QuantizedLinear.from_weight(synth_weight(256, 1024, seed=1).cuda())
+    x = synth_activation(rows, 1024, seed=2).cuda()
+    forms = [x, x.view(1, rows, 1024), lin.quantize_input(x)]
+    if rows <= 8:
+        forms.append(ops.pack(x, lin.high_bits_length, hadamard=True, sf_layout="rowmajor"))
+    for form in forms:
+        want = lin(form)
+        for shape, dtype in (((rows, 320), torch.bfloat16), ((rows + 1, 256), torch.bfloat16), ((rows, 256), torch.float16), ((rows * 256,), torch.bfloat16)):
+            bad = torch.full(shape, 7, dtype=dtype, device="cuda")
+            with pytest.raises((RuntimeError, TypeError)):
+                lin(form, out=bad)
+            assert bool((bad == 7).all())
+        with pytest.raises(RuntimeError):
+            lin(form, out=torch.empty(rows, 256, dtype=torch.bfloat16))
+        for ok in (torch.empty(rows, 256, dtype=torch.bfloat16, device="cuda"), torch.empty(rows, 1, 256, dtype=torch.bfloat16, device="cuda")):
+            got = lin(form, out=ok)
+            assert torch.equal(got, want) and got.data_ptr() == ok.data_ptr()
+    plq.check_device_status()
