@@ -279,10 +279,10 @@ def unpack_head_rows(k_rows: torch.Tensor, v_rows: torch.Tensor, t: int):
 
 
 def tile_scales(sf: torch.Tensor) -> torch.Tensor:
-    """Row-major scale bytes [rows, n] (contiguous, CUDA) -> the tiled layout, flat; padding is zero."""
+    """Row-major scale bytes [rows, n] (CUDA, any strides) -> the tiled layout, flat; padding is zero."""
     _require_cuda(sf, "sf")
     rows, n = sf.shape
-    sf = sf.to(torch.uint8)
+    sf = sf.to(torch.uint8).contiguous()          # the kernel takes rows of n neighbouring bytes
     L = _lib.lib()
     out = torch.empty(L.plq_sf_tiled_bytes(rows, n), dtype=torch.uint8, device=sf.device)
     with torch.cuda.device(sf.device):
