@@ -89,7 +89,11 @@ class _Layer:
 
 
 class ResQForwardB200:
-    """Decoder stack with packed weights resident on one GPU (one tensor-parallel rank)."""
+    """Decoder stack with packed weights resident on one GPU (one tensor-parallel rank).
+
+    `kv` holds the keys and values of each layer, [B, T, kv_heads, head_dim] (or packed rows).  What a caller keeps of it
+    stays as it is in later steps and shares no memory with them (a step that finds its cache held copies it).  After a
+    step behind a prompt the sequences of a batch may lie further apart than T rows: `.contiguous()` where that matters."""
 
     def __init__(self, cfg: LlamaConfig, device, ctx: Optional[tp.TPContext] = None, seed: int = 0,
                  num_layers: Optional[int] = None, fused_reduce_rows: int = 0, kv_quant: bool = False,
@@ -335,10 +339,10 @@ class ResQForwardB200:
         include the new rows, still to be written.  Returns (keys, values, first new row, rows allocated): the two are
         the leading positions of contiguous allocations.
 
-        Rows behind the views of `self.kv[li]` may be written in place only if these are the very tensors that the last
-        append made: then nobody else has a view of them.  Anything else - a prefill's cache, one restored from an
-        earlier step, one put there by the caller - is copied into a new allocation first, so every cache handed out
-        before keeps its contents."""
+        Rows behind the views of `self.kv[li]` are written in place only if these are the very tensors that the last
+        append made and nobody else holds them, a view of them or their storage.  Anything else - a prompt's cache, one
+        that the caller keeps from an earlier step, one put there by the caller - is copied into a new allocation first:
+        no two caches of different steps share memory."""
         width, dtype = (kv_cache.ROW_BYTES, torch.uint8) if self.kv_quant else (kv_cache.HEAD_DIM, torch.bfloat16)
         if len(self._kv_room) != len(self.layers):
             self._kv_room = [None] * len(self.layers)
@@ -349,21 +353,26 @@ class ResQForwardB200:
         k, v = self.kv[li]
         n, room = k.shape[1], self._kv_room[li]
         row = self.kv_heads * width
+
+        def extend(k, v, cap):                       # the first n + t of `cap` rows
+            size, stride = (b, n + t, self.kv_heads, width), (cap * row, row, width, 1)
+            k, v = self.kv[li] = k.as_strided(size, stride), v.as_strided(size, stride)
+            self._kv_room[li] = (weakref.ref(k), weakref.ref(v), cap)
+            return k, v
         if room is not None and room[0]() is k and room[1]() is v and n + t <= room[2] and k.shape[0] == b:
-            cap = room[2]
-        else:
-            for old in (k, v):
-                if old.dtype != dtype or tuple(old.shape) != (b, n, self.kv_heads, width):
-                    raise RuntimeError(f"the cache of layer {li} is {old.dtype} {tuple(old.shape)}, the new rows need "
-                                       f"{dtype} {(b, n, self.kv_heads, width)}")
-            cap = n + t + min(256, max(32, n // 8))  # one copy in that many steps instead of one in each
-            new = [torch.empty(b, cap, self.kv_heads, width, dtype=dtype, device=self.device) for _ in range(2)]
-            new[0][:, :n].copy_(k)
-            new[1][:, :n].copy_(v)
-            k, v = new
-        size, stride = (b, n + t, self.kv_heads, width), (cap * row, row, width, 1)
-        k, v = self.kv[li] = k.as_strided(size, stride), v.as_strided(size, stride)
-        self._kv_room[li] = (weakref.ref(k), weakref.ref(v), cap)
+            k, v = extend(k, v, room[2])             # the last reference of ours to the tensors without the new rows
+            if _lib.torch_lib().sharers(k) == 1 == _lib.torch_lib().sharers(v):
+                return k, v, n, room[2]
+            k, v = self.kv[li] = k[:, :n], v[:, :n]
+        for old in (k, v):
+            if old.dtype != dtype or tuple(old.shape) != (b, n, self.kv_heads, width):
+                raise RuntimeError(f"the cache of layer {li} is {old.dtype} {tuple(old.shape)}, the new rows need "
+                                   f"{dtype} {(b, n, self.kv_heads, width)}")
+        cap = n + t + min(256, max(32, n // 8))      # one copy in that many steps instead of one in each
+        new = [torch.empty(b, cap, self.kv_heads, width, dtype=dtype, device=self.device) for _ in range(2)]
+        new[0][:, :n].copy_(k)
+        new[1][:, :n].copy_(v)
+        k, v = extend(*new, cap)
         return k, v, n, cap
 
     def _gate_up(self, L: _Layer, pa: ops.PackedMatrix, like: int) -> ops.PackedMatrix:

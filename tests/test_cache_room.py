@@ -1,0 +1,106 @@
+"""Growing the key / value cache (host logic, on CPU tensors): rows are added in place only while nobody else holds the
+cache, and caches of different steps never share memory."""
+import types
+
+import pytest
+import torch
+
+from plaquant_b200 import forward_pass
+
+
+@pytest.fixture
+def model():
+    m = object.__new__(forward_pass.ResQForwardB200)
+    m.kv_quant, m.kv_heads, m.device, m.layers = False, 2, torch.device("cpu"), [types.SimpleNamespace()]
+    m.kv, m._kv_room = [None], []
+    return m
+
+
+def _append(m, b, t, pos0, value):
+    k, v, n, cap = m._cache_room(0, b, t, pos0)
+    assert n == pos0 and cap >= n + t and k.shape == v.shape == (b, n + t, 2, 128)
+    k[:, n:], v[:, n:] = value, -value
+
+
+def _check(cache, values):
+    for x, sign in zip(cache, (1, -1)):
+        assert x.shape[1] == len(values) and bool((x == sign * torch.tensor(values, dtype=x.dtype)[None, :, None, None]).all())
+
+
+HOLD = {"entry": lambda m: m.kv[0], "list": lambda m: list(m.kv), "tensor": lambda m: m.kv[0][1], "slice": lambda m: m.kv[0][0][:, :1],
+        "transposed": lambda m: m.kv[0][0].transpose(1, 2), "storage": lambda m: m.kv[0][1].untyped_storage(),
+        "numpy": lambda m: m.kv[0][0].view(torch.int16).numpy()}
+
+
+@pytest.mark.parametrize("mode", [torch.no_grad, torch.inference_mode, torch.enable_grad])
+@pytest.mark.parametrize("b", [1, 3])
+def test_steps_append_in_place_while_nobody_holds_the_cache(model, b, mode):
+    with mode():
+        _append(model, b, 5, 0, 1.0)
+        _append(model, b, 1, 5, 2.0)                      # behind a prompt: copied once
+        at = [x.data_ptr() for x in model.kv[0]]
+        values = [1.0] * 5 + [2.0]
+        for i in range(31):
+            _append(model, b, 1, 6 + i, 3.0 + i)
+            values.append(3.0 + i)
+            assert [x.data_ptr() for x in model.kv[0]] == at
+        _check(model.kv[0], values)
+        _append(model, b, 2, 37, 50.0)                    # past the spare rows
+        assert [x.data_ptr() for x in model.kv[0]] != at
+        _check(model.kv[0], values + [50.0] * 2)
+
+
+@pytest.mark.parametrize("mode", [torch.no_grad, torch.inference_mode])
+@pytest.mark.parametrize("how", sorted(HOLD))
+def test_a_held_cache_shares_no_memory_with_later_steps(model, how, mode):
+    with mode():
+        _append(model, 2, 3, 0, 1.0)
+        _append(model, 2, 1, 3, 2.0)
+        held = HOLD[how](model)
+        at = [x.data_ptr() for x in model.kv[0]]
+        _append(model, 2, 1, 4, 3.0)
+        moved = [x.data_ptr() for x in model.kv[0]]
+        assert not set(at) & set(moved)
+        _check(model.kv[0], [1.0] * 3 + [2.0, 3.0])
+        del held
+        _append(model, 2, 1, 5, 4.0)                      # nobody holds this one
+        assert [x.data_ptr() for x in model.kv[0]] == moved
+
+
+def test_editing_a_held_cache_changes_no_other(model):
+    _append(model, 2, 3, 0, 1.0)
+    _append(model, 2, 1, 3, 2.0)
+    first = list(model.kv)
+    _append(model, 2, 1, 4, 3.0)
+    second = list(model.kv)
+    first[0][0][:, 0] = 9.0                               # an older step's
+    _check(second[0], [1.0] * 3 + [2.0, 3.0])
+    second[0][1][:, 1] = 7.0                              # the live one: the next step continues from the edit
+    _append(model, 2, 1, 5, 4.0)
+    third = [x.clone() for x in model.kv[0]]
+    second[0][1].zero_()
+    assert all(torch.equal(x, y) for x, y in zip(third, model.kv[0])) and float(third[1][0, 1, 0, 0]) == 7.0
+    model.kv = first                                      # put back, edits included
+    _append(model, 2, 1, 4, 5.0)
+    assert float(model.kv[0][0][0, 0, 0, 0]) == 9.0 and float(first[0][0][1, 0, 0, 0]) == 9.0
+    assert first[0][0].shape[1] == 5                      # the caller's list follows the model
+
+
+def test_a_step_that_fails_leaves_the_cache(model, monkeypatch):
+    _append(model, 2, 3, 0, 1.0)
+    _append(model, 2, 1, 3, 2.0)
+    held = model.kv[0]
+
+    def no_memory(*a, **kw):
+        raise RuntimeError("out of memory")
+    monkeypatch.setattr(forward_pass.torch, "empty", no_memory)
+    with pytest.raises(RuntimeError):
+        model._cache_room(0, 2, 1, 4)
+    monkeypatch.undo()
+    _check(model.kv[0], [1.0] * 3 + [2.0])
+    _append(model, 2, 1, 4, 3.0)
+    _check(model.kv[0], [1.0] * 3 + [2.0, 3.0])
+    _check(held, [1.0] * 3 + [2.0])
+    with pytest.raises(RuntimeError):
+        model._cache_room(0, 3, 1, 5)                     # another batch size
+    _check(model.kv[0], [1.0] * 3 + [2.0, 3.0])
