@@ -94,6 +94,8 @@ class ResQForwardB200:
     `kv` holds the keys and values of each layer, [B, T, kv_heads, head_dim] (or packed rows).  What a caller keeps of it
     stays as it is in later steps and shares no memory with them (a step that finds its cache held copies it).  After a
     step behind a prompt the sequences of a batch may lie further apart than T rows: `.contiguous()` where that matters."""
+    _kv_room = ()                           # per layer: (weak references to the tensors of self.kv, rows allocated)
+    _rope_tables = None                     # both also for objects pickled before they existed
 
     def __init__(self, cfg: LlamaConfig, device, ctx: Optional[tp.TPContext] = None, seed: int = 0,
                  num_layers: Optional[int] = None, fused_reduce_rows: int = 0, kv_quant: bool = False,
@@ -136,7 +138,6 @@ class ResQForwardB200:
                 self.lm_head = (torch.randn(c.vocab_size, c.hidden_size, generator=g, device=self.device) * 0.02).to(torch.bfloat16)
         self.kv: List[Tuple[torch.Tensor, torch.Tensor]] = []
         self.pos = 0
-        self._kv_room: List[Optional[tuple]] = []        # per layer: (weak references to the tensors of self.kv, rows allocated)
         self._decode_states: Dict[tuple, _DecodeState] = {}
         # keys go into the cache as NVFP4 (Hadamard over the head dimension, per-head rows), queries get the same
         # rotation: the reference's QKRotationWrapper with k_had (promix/quantize/kv_quant.py:244-279)
@@ -262,7 +263,7 @@ class ResQForwardB200:
 
     def _rope_rows(self, pos0, t: int):
         """_rope_angles for the positions pos0 .. pos0 + t - 1 (the same values, from the tables where they reach)."""
-        if isinstance(pos0, int) and 0 <= pos0 and pos0 + t <= ROPE_TABLE_POSITIONS:
+        if self._rope_tables is not None and isinstance(pos0, int) and 0 <= pos0 and pos0 + t <= ROPE_TABLE_POSITIONS:
             return tuple(x[:, pos0:pos0 + t] for x in self._rope_tables)
         return self._rope_angles(torch.arange(pos0, pos0 + t, device=self.device, dtype=torch.float32))
 

@@ -29,6 +29,7 @@ SUPPORTED_FP_FORMATS = ("mxfp8", "nvfp4")
 
 class QuantizedLinear:
     """One mixed NVFP4 / MXFP8 linear layer: y = x @ W^T with both operands quantised."""
+    _native = None                  # also for objects pickled before it existed
 
     def __init__(self, w_main_int: torch.Tensor, w_main_scale: torch.Tensor,
                  w_high_int: Optional[torch.Tensor] = None, w_high_scale: Optional[torch.Tensor] = None,
@@ -48,7 +49,7 @@ class QuantizedLinear:
         self.grouped, self.groupsize, self.clip_ratio = grouped, groupsize, clip_ratio
         self.online_had, self.had_matrix = online_had, had_matrix
         self.gemm_impl = "b200"
-        self._gemm_w = self._gemv_w = self._native = None
+        self._gemm_w = self._gemv_w = None
         if w_main_int.is_cuda:
             self._prepare()
 

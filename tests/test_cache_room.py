@@ -86,6 +86,23 @@ def test_editing_a_held_cache_changes_no_other(model):
     assert first[0][0].shape[1] == 5                      # the caller's list follows the model
 
 
+def test_objects_pickled_by_an_earlier_version_still_work(model, monkeypatch):
+    """Their state has no native object, no cache room and no RoPE tables."""
+    from plaquant_b200 import ops, quantize
+    lin = object.__new__(quantize.QuantizedLinear)
+    lin.__dict__.update(_gemm_w="packed")
+    monkeypatch.setattr(ops, "native_linear", lambda w: ("native", w))
+    assert lin.native() == ("native", "packed") and lin.__getstate__()["_native"] is None
+    del model._kv_room
+    model.cfg = forward_pass.LlamaConfig()
+    _append(model, 2, 3, 0, 1.0)
+    _append(model, 2, 1, 3, 2.0)
+    _check(model.kv[0], [1.0] * 3 + [2.0])
+    want = model._rope_angles(torch.arange(5, 8, dtype=torch.float32))
+    assert all(torch.equal(x, y) for x, y in zip(model._rope_rows(5, 3), want))
+    assert len(object.__new__(forward_pass.ResQForwardB200)._kv_room) == 0
+
+
 def test_a_step_that_fails_leaves_the_cache(model, monkeypatch):
     _append(model, 2, 3, 0, 1.0)
     _append(model, 2, 1, 3, 2.0)
