@@ -95,7 +95,8 @@ class ResQForwardB200:
     stays as it is in later steps and shares no memory with them (a step that finds its cache held copies it).  After a
     step behind a prompt the sequences of a batch may lie further apart than T rows: `.contiguous()` where that matters."""
     _kv_room = ()                           # per layer: (weak references to the tensors of self.kv, rows allocated)
-    _rope_tables = None                     # both also for objects pickled before they existed
+    _rope_tables = _rope_for = None         # cos / sin rows, and the (theta, head size) they belong to; all three
+                                            # also for objects pickled before they existed
 
     def __init__(self, cfg: LlamaConfig, device, ctx: Optional[tp.TPContext] = None, seed: int = 0,
                  num_layers: Optional[int] = None, fused_reduce_rows: int = 0, kv_quant: bool = False,
@@ -144,7 +145,7 @@ class ResQForwardB200:
         self.kv_quant = kv_quant                     # False | True (packed NVFP4 rows in the cache) | "fake" (their bf16 values)
         if kv_quant and c.head_dim != 128:
             raise ValueError("kv_quant needs head_dim = 128 (one Hadamard block per head)")
-        self._rope_tables = self._rope_angles(torch.arange(ROPE_TABLE_POSITIONS, device=self.device, dtype=torch.float32))
+        self._make_rope_tables()
         torch.cuda.current_stream(self.device).synchronize()        # any stream may read them from here on
         # decode batches of up to `fused_reduce_rows` rows reduce over peer memory inside the RMSNorm-quant kernel
         self.peer = (tp.PeerReduce(fused_reduce_rows, c.hidden_size, self.device, self.ctx.group)
@@ -261,9 +262,15 @@ class ResQForwardB200:
         return (torch.cat([ang.cos(), ang.cos()], -1)[None, :, None, :],
                 torch.cat([ang.sin(), ang.sin()], -1)[None, :, None, :])
 
+    def _make_rope_tables(self) -> None:
+        self._rope_tables = self._rope_angles(torch.arange(ROPE_TABLE_POSITIONS, device=self.device, dtype=torch.float32))
+        self._rope_for = (self.cfg.rope_theta, self.cfg.head_dim)
+
     def _rope_rows(self, pos0, t: int):
-        """_rope_angles for the positions pos0 .. pos0 + t - 1 (the same values, from the tables where they reach)."""
-        if self._rope_tables is not None and isinstance(pos0, int) and 0 <= pos0 and pos0 + t <= ROPE_TABLE_POSITIONS:
+        """_rope_angles for the positions pos0 .. pos0 + t - 1 (the same values, from the tables where they reach and the
+        configuration is still the one they were made for)."""
+        if (self._rope_for == (self.cfg.rope_theta, self.cfg.head_dim) and isinstance(pos0, int) and 0 <= pos0
+                and pos0 + t <= ROPE_TABLE_POSITIONS):
             return tuple(x[:, pos0:pos0 + t] for x in self._rope_tables)
         return self._rope_angles(torch.arange(pos0, pos0 + t, device=self.device, dtype=torch.float32))
 

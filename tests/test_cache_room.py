@@ -103,6 +103,16 @@ def test_objects_pickled_by_an_earlier_version_still_work(model, monkeypatch):
     assert len(object.__new__(forward_pass.ResQForwardB200)._kv_room) == 0
 
 
+def test_rope_rows_follow_the_configuration(model):
+    model.cfg = forward_pass.LlamaConfig()
+    model._make_rope_tables()
+    for theta in (model.cfg.rope_theta, 10000.0):
+        model.cfg.rope_theta = theta
+        for pos0, t in ((0, 4), (5, 1), (32767, 1), (32766, 3)):
+            want = model._rope_angles(torch.arange(pos0, pos0 + t, dtype=torch.float32))
+            assert all(torch.allclose(x, y, rtol=0, atol=1e-6) for x, y in zip(model._rope_rows(pos0, t), want))
+
+
 def test_a_step_that_fails_leaves_the_cache(model, monkeypatch):
     _append(model, 2, 3, 0, 1.0)
     _append(model, 2, 1, 3, 2.0)
