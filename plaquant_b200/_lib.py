@@ -79,7 +79,7 @@ def torch_lib():
         except ImportError as e:
             raise RuntimeError("_plq_torch.so is missing or does not load: build it with `python -m plaquant_b200.build` "
                                "(there is no fallback path)") from e
-        _plq_torch.init(LIB_PATH)
+        _plq_torch.init(lib()._name)          # the library that is loaded, whatever LIB_PATH says by now
         _torch_lib = _plq_torch
     return _torch_lib
 

@@ -22,13 +22,14 @@ _kernel_loaded = False
 
 
 def init_kernel(path: Optional[str] = None, build_if_missing: bool = True):
-    """Loads libplq_b200.so (optionally from `path`); returns the ctypes handle."""
+    """Loads libplq_b200.so (optionally from `path`); returns the ctypes handle.  The PyTorch front end is this
+    package's own in either case."""
     global _kernel_loaded
     if path is not None:
         _lib.LIB_PATH = path
-    elif build_if_missing:
-        if build.needs_build():
-            build.build_library()
+    elif build_if_missing and build.needs_build():
+        build.build_library()
+    if build_if_missing:
         build.build_torch_front_end()
     handle = _lib.lib()
     _kernel_loaded = True

@@ -79,6 +79,18 @@ def test_torch_front_end_loads_and_leaves_cpu_tensors_to_the_caller(lib):
     assert lin.forward(torch.zeros(1, 256, dtype=torch.bfloat16), False, None, 1e-6, None) is None
 
 
+def test_front_end_belongs_to_the_loaded_library(lib, monkeypatch):
+    from plaquant_b200 import _lib, build, real_forward
+    monkeypatch.setattr(_lib, "_torch_lib", None)
+    monkeypatch.setattr(_lib, "LIB_PATH", "/nonexistent.so")          # changed after the library was loaded: no effect
+    assert _lib.torch_lib() is not None
+    built = []
+    monkeypatch.setattr(build, "build_torch_front_end", lambda *a: built.append(1))
+    monkeypatch.setattr(real_forward, "_kernel_loaded", False)
+    assert real_forward.init_kernel(path=lib._name) is lib and built == [1]      # a prebuilt library, a fresh checkout
+    assert real_forward.init_kernel(path=lib._name, build_if_missing=False) is lib and built == [1]
+
+
 def test_outputs_that_do_not_fit_are_refused():
     """Only the address and the row stride of `out` reach a kernel: every form that would be written past its end, between
     its elements or as another type is refused on the host."""

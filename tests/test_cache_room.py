@@ -110,6 +110,7 @@ def test_rope_rows_follow_the_configuration(model):
         model.cfg.rope_theta = theta
         for pos0, t in ((0, 4), (5, 1), (32767, 1), (32766, 3)):
             want = model._rope_angles(torch.arange(pos0, pos0 + t, dtype=torch.float32))
+            # one angle, two calls of cos: vector body and tail may differ by a few units of 2^-24
             assert all(torch.allclose(x, y, rtol=0, atol=1e-6) for x, y in zip(model._rope_rows(pos0, t), want))
 
 
