@@ -373,9 +373,9 @@ class ResQForwardB200:
                 return k, v, n, room[2]
             k, v = self.kv[li] = k[:, :n], v[:, :n]
         for old in (k, v):
-            if old.dtype != dtype or tuple(old.shape) != (b, n, self.kv_heads, width):
-                raise RuntimeError(f"the cache of layer {li} is {old.dtype} {tuple(old.shape)}, the new rows need "
-                                   f"{dtype} {(b, n, self.kv_heads, width)}")
+            if old.dtype != dtype or old.device != self.embed.device or tuple(old.shape) != (b, n, self.kv_heads, width):
+                raise RuntimeError(f"the cache of layer {li} is {old.dtype} {tuple(old.shape)} on {old.device}, the new rows need "
+                                   f"{dtype} {(b, n, self.kv_heads, width)} on {self.embed.device}")
         cap = n + t + min(256, max(32, n // 8))      # one copy in that many steps instead of one in each
         new = [torch.empty(b, cap, self.kv_heads, width, dtype=dtype, device=self.device) for _ in range(2)]
         new[0][:, :n].copy_(k)

@@ -12,7 +12,7 @@ from plaquant_b200 import forward_pass
 def model():
     m = object.__new__(forward_pass.ResQForwardB200)
     m.kv_quant, m.kv_heads, m.device, m.layers = False, 2, torch.device("cpu"), [types.SimpleNamespace()]
-    m.kv, m._kv_room = [None], []
+    m.kv, m._kv_room, m.embed = [None], [], torch.empty(0)
     return m
 
 
@@ -112,6 +112,15 @@ def test_rope_rows_follow_the_configuration(model):
             want = model._rope_angles(torch.arange(pos0, pos0 + t, dtype=torch.float32))
             # one angle, two calls of cos: vector body and tail may differ by a few units of 2^-24
             assert all(torch.allclose(x, y, rtol=0, atol=1e-6) for x, y in zip(model._rope_rows(pos0, t), want))
+
+
+def test_a_cache_that_does_not_belong_to_the_model_is_refused(model):
+    _append(model, 2, 3, 0, 1.0)
+    good = model.kv[0]
+    for bad in ([x.to("meta") for x in good], [x.float() for x in good], [x[:, :, :1] for x in good], [good[0], good[1][:, :2]], [x[:1] for x in good]):
+        model.kv = [tuple(bad)]
+        with pytest.raises(RuntimeError):
+            model._cache_room(0, 2, 1, 3)
 
 
 def test_a_step_that_fails_leaves_the_cache(model, monkeypatch):
