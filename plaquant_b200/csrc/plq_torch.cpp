@@ -173,7 +173,7 @@ std::tuple<Tensor, Tensor> decoder_layer(const Linear& qkv, const Linear& o, con
   TORCH_CHECK(h.is_contiguous() && h.scalar_type() == at::kBFloat16 && (!delta || (delta->is_contiguous() && delta->sizes() == h.sizes())),
               "h and delta must be contiguous bfloat16 [B, T, hidden]");
   TORCH_CHECK(qkv.n == nq && qkv.k() == hidden && o.k() == attn_width && o.n == hidden && gate_up.k() == hidden &&
-                  gate_up.n == 2 * ffn && down.n == hidden,
+                  gate_up.n == 2 * ffn && down.n == hidden && ffn % 128 == 0,
               "the layer's linears do not fit together");
   TORCH_CHECK(cos.numel() == t * 128 && sin.numel() == t * 128 && cos.is_contiguous() && sin.is_contiguous(), "cos / sin: one row per new position");
   const bool packed = k_view.scalar_type() == at::kByte;
@@ -188,8 +188,9 @@ std::tuple<Tensor, Tensor> decoder_layer(const Linear& qkv, const Linear& o, con
   const auto opts = h.options();
   // Workspace: the packed operand of the linear that runs, then its output; qkv's is dead before o's is written, and the
   // attention's operands have storage of their own.
+  const bool gated = rows > 16;                        // the GEMM applies SiLU(gate) * up itself: one column per pair
   const int64_t out0 = up256(2 * rows * hidden);
-  const Tensor ws = at::empty({packed_bytes + std::max(2 * rows * nq, out0 + 4 * rows * ffn)}, opts.dtype(at::kByte));
+  const Tensor ws = at::empty({packed_bytes + std::max(2 * rows * nq, out0 + (gated ? 2 : 4) * rows * ffn)}, opts.dtype(at::kByte));
   uint8_t* act = static_cast<uint8_t*>(ws.data_ptr()) + packed_bytes;
   void* stream = c10::cuda::getCurrentCUDAStream().stream();
   int32_t* status = qkv.status.data_ptr<int32_t>();
@@ -233,7 +234,6 @@ std::tuple<Tensor, Tensor> decoder_layer(const Linear& qkv, const Linear& o, con
   const int64_t out_rows = last_only ? b : rows;
   Tensor h2 = at::empty_like(h1), delta2 = at::empty_like(h1);
   uint8_t* gu = act + out0;
-  const bool gated = like > 16 && ffn % 128 == 0;      // the GEMM applies SiLU(gate) * up itself
   {
     const PackedAt p(ws.data_ptr(), out_rows, o.k_lo, o.k_hi);
     check(api.pack(attn.const_data_ptr(), out_rows, attn_width, o.k_hi, 1, p.lo, p.lo_sf, p.hi, p.hi_sf, PLQ_SF_TILED, stream));

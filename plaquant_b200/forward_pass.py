@@ -385,10 +385,12 @@ class ResQForwardB200:
 
     def _gate_up(self, L: _Layer, pa: ops.PackedMatrix, like: int) -> ops.PackedMatrix:
         """down_proj's packed input: gate_up, SiLU(gate) * up, rotation, quantisation.  Batches on the GEMM (more than 16
-        rows in the whole pass) get the activation from the product's own epilogue."""
-        if like > 16 and type(L.gate_up) is QuantizedLinear and self.ffn % 128 == 0 and L.gate_up._gemm_w is not None:
-            return ops.pack(ops.mixed_gemm_silu_mul(pa, L.gate_up._gemm_w), self.k_hi_ffn, hadamard=True)
-        gu = L.gate_up(pa)                                                              # [rows, 2 * ffn] = [gate | up]
+        rows in the whole pass, `like`, however few of them are left in `pa`) get the activation from the product's own
+        epilogue; other linears than the package's own, or one switched to another product, are called."""
+        lin = L.gate_up                              # ffn is a multiple of 128 (down_proj's rotation)
+        if like > 16 and type(lin) is QuantizedLinear and lin.gemm_impl == "b200" and lin._gemm_w is not None:
+            return ops.pack(ops.mixed_gemm_silu_mul(pa, lin._gemm_w), self.k_hi_ffn, hadamard=True)
+        gu = lin(pa)                                                                    # [rows, 2 * ffn] = [gate | up]
         return ops.silu_mul_pack(gu, self.k_hi_ffn)
 
     def _plain_layer(self, L: _Layer) -> bool:

@@ -141,3 +141,13 @@ def test_a_step_that_fails_leaves_the_cache(model, monkeypatch):
     with pytest.raises(RuntimeError):
         model._cache_room(0, 3, 1, 5)                     # another batch size
     _check(model.kv[0], [1.0] * 3 + [2.0, 3.0])
+
+
+def test_a_gate_up_switched_to_another_product_is_refused(model):
+    """The activation in the product's epilogue takes the same linears as the call it replaces."""
+    from plaquant_b200 import quantize
+    lin = object.__new__(quantize.QuantizedLinear)
+    lin.__dict__.update(gemm_impl="pytorch", _gemm_w=types.SimpleNamespace(rows=256))
+    model.ffn, model.k_hi_ffn = 128, 0
+    with pytest.raises(ValueError):
+        model._gate_up(types.SimpleNamespace(gate_up=lin), None, like=100)
