@@ -260,8 +260,11 @@ std::tuple<Tensor, Tensor> decoder_layer(const Linear& qkv, const Linear& o, con
   return {h2, delta2};
 }
 
-// How many tensors share t's memory, t included; the base that a view keeps alive does not count.
-int64_t sharers(const Tensor& t) { return static_cast<int64_t>(t.storage().use_count()) - (t.is_view() ? 1 : 0); }
+// Does nothing else share the memory of a or of b?  (The base that a view keeps alive does not count.)
+bool alone(const Tensor& a, const Tensor& b) {
+  auto one = [](const Tensor& t) { return t.storage().use_count() == (t.is_view() ? 2u : 1u); };
+  return one(a) && one(b);
+}
 
 }  // namespace
 
@@ -273,6 +276,6 @@ PYBIND11_MODULE(_plq_torch, m) {
       .def("forward", &Linear::forward);
   m.def("init", &init);
   m.def("pack", &pack);
-  m.def("sharers", &sharers);
+  m.def("alone", &alone);
   m.def("decoder_layer", &decoder_layer);
 }

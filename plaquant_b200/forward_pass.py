@@ -362,15 +362,13 @@ class ResQForwardB200:
         n, room = k.shape[1], self._kv_room[li]
         row = self.kv_heads * width
 
-        def extend(k, v, cap):                       # the first n + t of `cap` rows
-            size, stride = (b, n + t, self.kv_heads, width), (cap * row, row, width, 1)
-            k, v = self.kv[li] = k.as_strided(size, stride), v.as_strided(size, stride)
-            self._kv_room[li] = (weakref.ref(k), weakref.ref(v), cap)
-            return k, v
         if room is not None and room[0]() is k and room[1]() is v and n + t <= room[2] and k.shape[0] == b:
-            k, v = extend(k, v, room[2])             # the last reference of ours to the tensors without the new rows
-            if _lib.torch_lib().sharers(k) == 1 == _lib.torch_lib().sharers(v):
-                return k, v, n, room[2]
+            cap = room[2]                            # k and v, the first n + t rows from here on, were our last reference
+            size, stride = (b, n + t, self.kv_heads, width), (cap * row, row, width, 1)     # to the tensors without the new ones
+            k, v = self.kv[li] = k.as_strided(size, stride), v.as_strided(size, stride)
+            if _lib.torch_lib().alone(k, v):
+                self._kv_room[li] = (weakref.ref(k), weakref.ref(v), cap)
+                return k, v, n, cap
             k, v = self.kv[li] = k[:, :n], v[:, :n]
         for old in (k, v):
             if old.dtype != dtype or old.device != self.embed.device or tuple(old.shape) != (b, n, self.kv_heads, width):
@@ -380,7 +378,9 @@ class ResQForwardB200:
         new = [torch.empty(b, cap, self.kv_heads, width, dtype=dtype, device=self.device) for _ in range(2)]
         new[0][:, :n].copy_(k)
         new[1][:, :n].copy_(v)
-        k, v = extend(*new, cap)
+        size, stride = (b, n + t, self.kv_heads, width), (cap * row, row, width, 1)
+        k, v = self.kv[li] = new[0].as_strided(size, stride), new[1].as_strided(size, stride)
+        self._kv_room[li] = (weakref.ref(k), weakref.ref(v), cap)
         return k, v, n, cap
 
     def _gate_up(self, L: _Layer, pa: ops.PackedMatrix, like: int) -> ops.PackedMatrix:
