@@ -351,11 +351,14 @@ PLQ_API int plq_gemv_static_scratch(const void* a_lo_codes, const void* a_lo_sf,
  * (weight codes and scales) was complete before the kernels that precede this call in the stream
  * were launched - true for weights packed at load time, not for a weight packed by the call just
  * before - and the first weight loads are issued before that wait (about 10 % on the largest
- * decode shape).  `dev_status` as for plq_mixed_gemm.
+ * decode shape).  PLQ_GEMV_INTERLEAVED says that other kernels (a pack, a norm) run between this and
+ * the next such call on the stream: a hint for the choice of the ring, without influence on results.
+ * `dev_status` as for plq_mixed_gemm.
  * Replaces the same reference lines as plq_gemv (the quantised linear at decode batch sizes,
  * promix/quantize/quant_utils.py:389 / inference/forward_pass.py:319).
  */
 #define PLQ_GEMV_STATIC_B 1   /* flags: the B operand is never written by the kernels just before the call */
+#define PLQ_GEMV_INTERLEAVED 2   /* flags: the launches before and after this one are not GEMVs */
 PLQ_API int plq_gemv_tc(const void* a_lo_codes, const void* a_lo_sf, const void* a_hi_codes, const void* a_hi_sf,
                         const void* b_lo_codes, const void* b_lo_sf, const void* b_hi_codes, const void* b_hi_sf,
                         int64_t m, int64_t n, int64_t k_lo, int64_t k_hi,

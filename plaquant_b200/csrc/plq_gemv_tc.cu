@@ -454,16 +454,29 @@ static int gt_launch_planned(const GtMaps& tm, const GtArgs& g, int slices, int 
 }
 
 template <int MR>
-static int gt_launch(const GtMaps& tm, const GtArgs& g, int64_t n, int64_t k_lo, int64_t k_hi, cudaStream_t stream) {
+static int gt_launch(const GtMaps& tm, const GtArgs& g, int64_t n, int64_t k_lo, int64_t k_hi, bool interleaved, cudaStream_t stream) {
   int slices = 1, grid = 1;
   if (gt_max_clusters<MR, kGtStagesShared>(1) < 1) return PLQ_ERR_CUDA;     // also sets the kernel's shared-memory attribute
   gt_plan<MR>(n, k_lo, k_hi, sm_count(), &slices, &grid);
-  // A grid of at most one CTA per SM has the SM's shared memory to itself: a ring twice as deep, where a CTA has more
-  // stages than the shallow one holds (all clusters must still be resident at once).  Replayed alone, m = 16: 14336 -> 4096
-  // 11.5 -> 10.4 us, 4096 -> 6144 7.1 -> 6.6, m = 8: 4096 -> 4096 (five stages) 4.85 -> 5.5, the next GEMV losing its early
-  // start; between the other kernels of a decode step it is faster there too (16 layers, m = 2: 40.1 -> 39.3 ms in 16 steps).
-  const int64_t k_stages = g.lo_stages + g.hi_stages;
-  if (grid <= sm_count() && (k_stages + slices - 1) / slices > kGtStagesShared && gt_max_clusters<MR, kGtStagesAlone>(slices) * slices >= grid)
+  // A grid of at most one CTA per SM can have a ring twice as deep (all clusters must still be resident at once); it pays
+  // where a CTA has more stages than the shallow ring holds.  Its CTAs fill the SMs' shared memory, though, and a GEMV right
+  // behind this one loses its early start: that is worse where most SMs are taken (more than 2/3) and a CTA streams for a
+  // short time only (11 stages; 13 where next to all are taken).  A caller whose launches have other kernels between them says so (PLQ_GEMV_INTERLEAVED): it
+  // then still pays with m <= 8, or whole tiles per CTA, as long as an eighth of the SMs is left for the neighbours.  Shallow ->
+  // deep ring, us, replayed over rotating weights back to back / with a pack in front of each (CTAs x stages per CTA):
+  //   4096 -> 4096 m = 8 (128 x 5) 4.91 -> 5.54 / 6.51 -> 6.34       8192 -> 4096 m = 8 (128 x 9) 6.80 -> 7.31 / 8.48 -> 8.41
+  //   4096 -> 8192 m = 16 (128 x 9) 7.45 -> 7.72 / 8.93 -> 8.99      8192 -> 8192 m = 16 (128 x 17) 10.87 -> 10.14 / 12.45 -> 12.22
+  //   7168 -> 5120 m = 16 (120 x 10) 7.64 -> 7.66 / 9.76 -> 9.93     4096 -> 6144 m = 16 (96 x 9) 7.14 -> 6.61 / 8.43 -> 8.02
+  //   2048 -> 14336 m = 8 (112 x 9) 5.66 -> 5.88 / 7.71 -> 7.06      3072 -> 14336 m = 8 (112 x 13) 7.67 -> 7.08 / 9.52 -> 8.53
+  //   2048 -> 18944 m = 16 (148 x 9) 6.90 -> 7.25 / 8.23 -> 8.61     3072 -> 18944 m = 16 (148 x 13) 8.60 -> 8.61 / 9.99 -> 10.29
+  //   4096 -> 18944 m = 16 (148 x 17) 10.39 -> 9.84 / 12.09 -> 11.89
+  const int sms = sm_count();
+  const int64_t cta_stages = (g.lo_stages + g.hi_stages + slices - 1) / slices;
+  const bool full = 8 * grid > 7 * sms;
+  const bool crowded = 3 * grid > 2 * sms && cta_stages <= (full ? 13 : 11);
+  const bool neighbours_fit = interleaved && (MR == 8 || slices == 1) && !full;
+  const bool deep = grid <= sms && cta_stages > kGtStagesShared && (!crowded || neighbours_fit);
+  if (deep && gt_max_clusters<MR, kGtStagesAlone>(slices) * slices >= grid)
     return gt_launch_planned<MR, kGtStagesAlone>(tm, g, slices, grid, stream);
   return gt_launch_planned<MR, kGtStagesShared>(tm, g, slices, grid, stream);
 }
@@ -518,8 +531,9 @@ extern "C" int plq_gemv_tc(const void* a_lo_codes, const void* a_lo_sf, const vo
     if ((st = make_sf_tmap(&tm.sfw_hi, b_hi_sf, g.hi_stages, groups, 1)) != PLQ_OK) return st;
     if ((st = make_sf_tmap(&tm.sfx_hi, a_hi_sf, g.hi_stages, 1, 1)) != PLQ_OK) return st;
   }
-  return m <= 8 ? gt_launch<8>(tm, g, n, k_lo, k_hi, static_cast<cudaStream_t>(stream))
-                : gt_launch<16>(tm, g, n, k_lo, k_hi, static_cast<cudaStream_t>(stream));
+  const bool interleaved = (flags & PLQ_GEMV_INTERLEAVED) != 0;
+  return m <= 8 ? gt_launch<8>(tm, g, n, k_lo, k_hi, interleaved, static_cast<cudaStream_t>(stream))
+                : gt_launch<16>(tm, g, n, k_lo, k_hi, interleaved, static_cast<cudaStream_t>(stream));
 }
 
 #ifdef PLQ_GEMV_TRACE

@@ -119,9 +119,9 @@ struct Linear {
   // `like`: the choice of kernel for another number of rows (the two sum K in different orders).
   int product(const PackedAt& a, int64_t rows, void* y, int64_t ldy, void* stream, int64_t like = 0) const {
     int32_t* st = status.data_ptr<int32_t>();
-    if (std::max(rows, like) <= 16)      // decode: stream the weights once
+    if (std::max(rows, like) <= 16)      // decode: stream the weights once; every product here has a pack in front of it
       return api.gemv_tc(a.lo, a.lo_sf, a.hi, a.hi_sf, ptr(lo), ptr(lo_sf), ptr(hi), ptr(hi_sf), rows, n, k_lo, k_hi, y, ldy, st,
-                         PLQ_GEMV_STATIC_B, stream);
+                         PLQ_GEMV_STATIC_B | PLQ_GEMV_INTERLEAVED, stream);
     return api.mixed_gemm(a.lo, a.lo_sf, a.hi, a.hi_sf, ptr(lo), ptr(lo_sf), ptr(hi), ptr(hi_sf), rows, n, k_lo, k_hi, y, ldy, st,
                           stream);
   }

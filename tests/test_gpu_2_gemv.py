@@ -99,6 +99,25 @@ def test_llama8b_shapes_gemv_tc(n, k, m):
     assert rel_l2(f32_of(y)[:, sel], want) <= TOL
 
 
+# CTAs per launch x stages per CTA on both sides of every line of the ring's rule (m <= 8): 64 x 4 (the shallow ring holds it),
+# 64 x 5, 128 x 5 and x 15 in clusters of four, 128 x 8 and x 15 in pairs, 120 x 6 in threes, 96 x 9, 112 x 9, 148 x 9, more tiles than SMs
+@pytest.mark.parametrize("n,k", [(2048, 3072), (2048, 4096), (4096, 4096), (4096, 14336), (8192, 3584), (8192, 7168), (5120, 4096),
+                                 (6144, 4096), (14336, 2048), (18944, 2048), (19072, 2048)])
+@pytest.mark.parametrize("m", [8, 9])
+def test_ring_depth_has_no_influence_on_results(n, k, m):
+    k_hi = k // 32 // 64 * 64
+    xc, wc = synth_activation(m, k, seed=m).cuda(), synth_weight(n, k, seed=n + k).cuda()
+    pa, pb = (plq.pack(t, k_hi, hadamard=True, sf_layout="tiled") for t in (xc, wc))
+    torch.cuda.synchronize()
+    y = plq.gemv_tc(pa, pb)
+    for static in (False, True):
+        for _ in range(3):                                  # one behind the other: early starts included
+            again = plq.gemv_tc(pa, pb, static_weights=static, interleaved=True)
+            assert torch.equal(y, again)
+    plq.check_device_status()
+    assert rel_l2(f32_of(y), f32_of(plq.mixed_gemm(pa, pb))) <= TOL
+
+
 def test_gemv_tc_argument_errors():
     x = synth_activation(17, 256, seed=1).cuda()
     pa = plq.pack(x, 64, sf_layout="tiled")
