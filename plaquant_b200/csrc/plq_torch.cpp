@@ -158,6 +158,7 @@ Tensor heads_first(const Tensor& t) { return t.transpose(1, 2); }
 // One decoder layer on one GPU: h + delta -> RMSNorm(ln1) -> qkv -> RoPE, cache append -> attention -> o_proj -> residual,
 // RMSNorm(ln2) -> gate_up -> SiLU * up -> down_proj.  Returns (residual stream, down_proj's output not added to it yet).
 // k_view / v_view: the first `ctx` positions of caches allocated for `cap`; the new rows go to `pos` (or *pos_dev).
+// More than one position per sequence: all of them (a causal mask over the positions themselves) or with a mask.
 // Packed caches (uint8) need `had`, the float32 Hadamard of the queries.  With `last_only` everything behind the attention
 // runs for the last position of each sequence alone, results [B, 1, hidden] (the same bits: rows are independent).
 std::tuple<Tensor, Tensor> decoder_layer(const Linear& qkv, const Linear& o, const Linear& gate_up, const Linear& down,
@@ -183,6 +184,7 @@ std::tuple<Tensor, Tensor> decoder_layer(const Linear& qkv, const Linear& o, con
                     c->scalar_type() == k_view.scalar_type() && (b == 1 || c->stride(0) == cap * kv_heads * width) &&
                     c->stride(1) == kv_heads * width && c->stride(2) == width && c->stride(3) == 1,
                 "the caches must be the leading positions of contiguous allocations");
+  TORCH_CHECK(t == 1 || mask || t == ctx, "a chunk behind a prompt needs a mask");
   int64_t packed_bytes = 0;
   for (const Linear* l : {&qkv, &o, &gate_up, &down}) packed_bytes = std::max(packed_bytes, l->packed_bytes(rows));
   const auto opts = h.options();

@@ -5,11 +5,17 @@ import types
 import pytest
 import torch
 
-from plaquant_b200 import forward_pass
+from plaquant_b200 import build, forward_pass
+
+
+@pytest.fixture(scope="module")
+def front_end():
+    build.build_library()
+    build.build_torch_front_end()
 
 
 @pytest.fixture
-def model():
+def model(front_end):
     m = object.__new__(forward_pass.ResQForwardB200)
     m.kv_quant, m.kv_heads, m.device, m.layers = False, 2, torch.device("cpu"), [types.SimpleNamespace()]
     m.kv, m._kv_room, m.embed = [None], [], torch.empty(0)
@@ -151,3 +157,20 @@ def test_a_gate_up_switched_to_another_product_is_refused(model):
     model.ffn, model.k_hi_ffn = 128, 0
     with pytest.raises(ValueError):
         model._gate_up(types.SimpleNamespace(gate_up=lin), None, like=100)
+
+
+@pytest.mark.parametrize("mask_elements", [1 << 27, 0])
+@pytest.mark.parametrize("b,t,ctx,heads", [(2, 1, 7, 4), (2, 5, 5, 2), (1, 2, 3, 4), (3, 5, 12, 2), (1, 64, 200, 2)])
+def test_a_chunk_sees_every_position_before_it(model, monkeypatch, b, t, ctx, heads, mask_elements):
+    """Query i of a chunk is position ctx - t + i: attention over that many positions and itself, in float64."""
+    monkeypatch.setattr(forward_pass, "CHUNK_MASK_ELEMENTS", mask_elements)
+    model.heads, model.cfg = heads, forward_pass.LlamaConfig()
+    g = torch.Generator().manual_seed(t)
+    q, kk, vv = (torch.randn(b, n, h, 128, generator=g).to(torch.bfloat16) for n, h in ((t, heads), (ctx + 3, 2), (ctx + 3, 2)))
+    got = model._attend(q, kk, vv, ctx, None).view(b, t, heads, 128)
+    qd, kd, vd = q.double(), kk[:, :ctx].double().repeat_interleave(heads // 2, 2), vv[:, :ctx].double().repeat_interleave(heads // 2, 2)
+    w = torch.einsum("bthd,bshd->bhts", qd, kd) / 128 ** 0.5
+    w = w.masked_fill(torch.arange(ctx)[None] > torch.arange(ctx - t, ctx)[:, None], float("-inf")).softmax(-1)
+    want = torch.einsum("bhts,bshd->bthd", w, vd)
+    # bf16 probabilities and results: two roundings of 2^-9 each, probabilities summed over values up to 5
+    assert (got.double() - want).abs().max() <= 2.0 ** -9 * (want.abs().max() + vd.abs().max())

@@ -1,4 +1,4 @@
-"""The native calls that take a whole linear or half a decoder layer: the same kernels on the same operands as the
+"""The native calls that take a whole linear or a decoder layer: the same kernels on the same operands as the
 operator-by-operator path, so every result is compared bit for bit with that path."""
 import copy
 import pickle
@@ -47,7 +47,7 @@ def test_linear_call_equals_pack_and_product(rows, k, n, k_hi_fraction):
 @pytest.mark.parametrize("head_dim,heads,kv_heads,kv_quant", [(128, 4, 2, False), (128, 4, 1, True), (128, 4, 4, "fake"),
                                                               (64, 4, 2, False), (128, 18, 2, False)])
 def test_layer_calls_equal_the_operator_path(monkeypatch, head_dim, heads, kv_heads, kv_quant):
-    """Prompt, a chunk behind it, single steps, graph decode; 18 heads over 2 key heads: no decode-attention kernel."""
+    """Prompt, a chunk behind it, single steps, graph decode; also 9 query heads per key head."""
     from plaquant_b200 import forward_pass
     cfg = forward_pass.LlamaConfig(hidden_size=heads * head_dim, intermediate_size=1024, num_layers=2, num_heads=heads,
                                    num_kv_heads=kv_heads, head_dim=head_dim, vocab_size=400)
@@ -124,4 +124,32 @@ def test_linear_refuses_an_output_that_does_not_fit(rows):
         for ok in (torch.empty(rows, 256, dtype=torch.bfloat16, device="cuda"), torch.empty(rows, 1, 256, dtype=torch.bfloat16, device="cuda")):
             got = lin(form, out=ok)
             assert torch.equal(got, want) and got.data_ptr() == ok.data_ptr()
+    plq.check_device_status()
+
+
+@pytest.mark.parametrize("mask_elements", [1 << 27, 0])
+@pytest.mark.parametrize("kv_quant", [False, True, "fake"])
+@pytest.mark.parametrize("head_dim,heads,kv_heads", [(128, 4, 2), (64, 4, 4)])
+def test_a_prompt_in_chunks_attends_like_the_whole_prompt(monkeypatch, head_dim, heads, kv_heads, kv_quant, mask_elements):
+    """One layer, so that no later layer's 4-bit inputs amplify a rounding: the attention of a chunk behind a prompt against
+    those rows of the whole prompt's attention, on the same projections."""
+    from plaquant_b200 import forward_pass
+    if kv_quant and head_dim != 128:
+        pytest.skip("packed caches have heads of 128")
+    monkeypatch.setattr(forward_pass, "CHUNK_MASK_ELEMENTS", mask_elements)
+    cfg = forward_pass.LlamaConfig(hidden_size=heads * head_dim, intermediate_size=256, num_layers=1, num_heads=heads,
+                                   num_kv_heads=kv_heads, head_dim=head_dim, vocab_size=100)
+    m = forward_pass.ResQForwardB200(cfg, "cuda", seed=3, kv_quant=kv_quant)
+    qkv = torch.randn(2, 300, (heads + 2 * kv_heads) * head_dim, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16).cuda()
+    m.kv = [None]
+    whole = m._attention(0, qkv, 0, m._rope_rows(0, 300), None)
+    m.kv = [None]
+    parts = [m._attention(0, qkv[:, a:b].contiguous(), a, m._rope_rows(a, b - a), None) for a, b in ((0, 100), (100, 102), (102, 299), (299, 300))]
+    got = torch.cat(parts, 1)
+    # bf16 results of float32 sums in another order: one step, 2^-8 of the largest
+    assert (got.float() - whole.float()).abs().max() <= 2.0 ** -8 * whole.float().abs().max()
+    assert m.kv[0][0].shape[1] == 300
+    ids = torch.randint(0, 100, (2, 40), generator=torch.Generator().manual_seed(6)).cuda()
+    m.forward(ids[:, :20])
+    assert torch.isfinite(m.forward(ids[:, 20:], pos0=20, all_positions=True)).all()
     plq.check_device_status()
