@@ -139,8 +139,8 @@ __device__ __forceinline__ float e8m0_to_f32(uint32_t code) { return __uint_as_f
 // SiLU(g) = g / (1 + exp(-g)) of a bf16-valued g, to be rounded to bf16 by the caller.  The CPU oracle defines it
 // with a float32 exponential written down operation by operation and an IEEE division (silu_mul_bf16 / exp_det); the
 // value needed is its rounding to 8 significant bits for one of 65 280 possible inputs, and the hardware's ex2 and
-// rcp approximations (a few units in the 24th bit) give the same bf16 for every one of them - the GPU tests compare
-// all finite inputs - with 5 instructions per element instead of the definition's ~35 ([32768, 28672] -> packed:
+// rcp approximations (a few units in the 24th bit) give the same bf16 for every one of them - two GPU tests compare all
+// finite inputs, test_silu_of_every_bf16_value_bit_exact and test_silu_of_the_smallest_values_bit_exact - with 5 instructions per element instead of the definition's ~35 ([32768, 28672] -> packed:
 // 2175 -> 890 us = 4.8 TB/s).
 // The denominator is scaled by 1/4: up to 2^126 its reciprocal is a normal number, above that exp has overflowed and
 // the quotient is zero on either path.
