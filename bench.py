@@ -232,7 +232,7 @@ def config_dict(n_gpus):
 
 
 def cpu_model_estimate(budget_s: float = 8.0):
-    """configs[4] on the host, extrapolated: the CPU arm's code on 64 token rows x 1024 weight rows of each of the
+    """The decoder workload on the host, extrapolated: the CPU arm's code on 64 token rows x 1024 weight rows of each of the
     four linears of one Llama-3-70B decoder layer (full K), and from its rate the tokens/s the 80 layers' linears
     alone would allow (a full 70B forward does not fit a host's memory or a benchmark's time)."""
     import torch
@@ -475,7 +475,7 @@ def main_ours(args, rank, local_rank, world):
 
 
 def run_model_tp(args, torch, plq, rank, world, dev, peaks):
-    """configs[4] on the ranks of this run: the Llama-3-70B-architecture decoder stack (random init, `--tp-layers`
+    """The decoder workload on the ranks of this run: the Llama-3-70B-architecture decoder stack (random init, `--tp-layers`
     of its 80 layers), tensor-parallel over the N ranks (column-parallel QKV / gate_up, row-parallel O / down, one
     reduction per row-parallel linear, done inside the following RMSNorm-quant kernel over peer memory: all-reduce
     form for decode batches, reduce-scatter + all-gather of the packed rows for the prefill),
@@ -586,7 +586,7 @@ def run_model_tp(args, torch, plq, rank, world, dev, peaks):
 
 
 def main_model(args, rank, local_rank, world):
-    """random-init Llama-3-70B-architecture decoder stack, tensor-parallel over the ranks
+    """Random-init Llama-3-70B-architecture decoder stack, tensor-parallel over the ranks
     (column-parallel QKV / gate_up, row-parallel O / down, one NCCL all-reduce after each row-parallel
     linear), batch 16, prefill of 2048 random token ids + 128 greedy decode steps.  Strong scaling:
     the job is fixed, the ranks share it."""
@@ -710,8 +710,8 @@ def time_rotating(torch, fns, rounds):
 
 
 def side_benchmarks(plq, torch, dev, peaks):
-    """configs[1] (fused RMSNorm-quant + Hadamard-pack, [4096, 4096]) and configs[2] (decode GEMV
-    sweep), each kernel timed alone with an L2 flush before every launch; HBM roofline."""
+    """Fused RMSNorm-quant + Hadamard-pack, [4096, 4096], and the decode GEMV sweep,
+    each kernel timed alone with an L2 flush before every launch; HBM roofline."""
     flush = torch.zeros(256 * 1024 * 1024 // 4, dtype=torch.int32, device=dev)     # 256 MB > L2
     out = {}
     g = torch.Generator().manual_seed(77)

@@ -94,8 +94,9 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
 }
 
 // Work item `v` of a launch -> its row tile, first column and whether it is half a tile wide.  The items of a last wave
-// that would leave most of the CTA pairs idle are halved (256 x 128, one MMA of N = 128 per K step): 333 x 28672 has 224
-// tiles for 74 pairs, and the two left over after three waves cost a fourth of the time of a whole wave.
+// that would leave most of the CTA pairs idle are halved (256 x 128, one MMA of N = 128 per K step): 1024 x 6144 has 96
+// tiles for 74 pairs, and the 22 left over after the first wave would take as long as it; as 44 halves they take 0.8 of that
+// (K = 4096: 26.6 -> 24.6 us).
 template <int BN, int CG>
 struct WorkItem {
   int tm, n0;

@@ -36,9 +36,19 @@ namespace plq {
 constexpr int kPackTargetThreads = PLQ_PACK_TARGET_THREADS;   // CTA size the launcher aims for (whole rows)
 // Rotated rows go to pack_rows_kernel up to this many of its warps per SM: one resident set (64) with a norm alone, whose
 // warps wait for each other; two where a residual is added or nothing is; four with SiLU.  Replayed, this kernel against
-// pack_kernel, us: m = 16, K = 4096 norm 2.4 / 4.0, residual + norm 2.6 / 4.5; m = 333 norm 4.0 / 5.2; 8192 x 512 (55 warps
-// per SM) norm 7.3 / 7.1; 4096 x 2048 (111) plain 7.7 / 8.8, SiLU 10.4 / 12.6, norm 10.7 / 10.6, residual + norm 13.7 / 15.0;
-// 4096 x 4096 (221) plain 13.9 / 13.4, SiLU 19.1 / 21.2, residual + norm 27.0 / 26.9.
+// pack_kernel, us, at so many warps per SM (m = 16, K = 4096: norm 2.4 / 4.0, residual + norm 2.6 / 4.5):
+//                      48            64            80            96            112           128           224           256
+//   plain, K = 4096    4.8 / 5.5     4.9 / 5.3     5.9 / 5.5     6.8 / 7.1     7.6 / 8.7     8.4 / 9.2    13.5 / 13.1   15.2 / 14.3
+//   plain, K = 14336   4.8 / 5.2     4.9 / 5.4     5.9 / 5.5     6.8 / 7.3     7.5 / 8.5     8.4 / 8.6    13.3 / 11.8   15.0 / 12.9
+//   norm, K = 4096     5.9 / 7.6     6.7 / 6.6     8.0 / 9.5     9.6 / 10.7   10.7 / 10.4   12.0 / 10.6   19.3 / 18.2   21.7 / 18.6
+//   norm, K = 8192     5.9 / 7.0     7.4 / 7.3     8.9 / 9.8    10.4 / 10.6   11.9 / 10.8   13.4 / 10.8   22.3 / 18.3   25.3 / 18.4
+//   add + norm, 4096   7.0 / 9.2     8.5 / 9.5    10.5 / 13.9   11.8 / 14.8   13.7 / 14.7   15.2 / 15.2   27.2 / 27.1   31.1 / 29.3
+//   add + norm, 8192   7.4 / 8.6     9.2 / 12.2   11.2 / 12.5   13.1 / 12.8   15.1 / 16.4   16.9 / 16.8   30.1 / 26.7   35.3 / 30.7
+//   SiLU, K = 4096     6.4 / 6.4     6.5 / 7.2     8.0 / 10.5    9.2 / 12.3   10.4 / 12.3   11.6 / 12.5   19.1 / 21.3   21.6 / 23.7
+//   SiLU, K = 14336    6.4 / 6.4     6.6 / 7.4     8.0 / 10.3    9.2 / 11.7   10.3 / 11.9   11.5 / 12.0   18.8 / 19.5   21.3 / 21.7
+// pack_kernel's steps are its waves.  Inside the limits it is ahead by 8 % just past one set of plain rows (80) and by up to 2 %
+// at the end of the norm's (64) and once with a residual (96, K = 8192), level or behind everywhere else.  K <= 1024 is faster
+// here far beyond the limits (K = 512, 256 warps per SM: plain 14.5 / 41.6, norm 39.7 / 57.2); the rule does not look at K.
 constexpr int pack_rows_warps(int pro, bool norm) { return pro == 1 ? 256 : norm && pro == 0 ? 64 : 128; }
 
 struct PackArgs {

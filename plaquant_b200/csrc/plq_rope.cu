@@ -153,7 +153,7 @@ __device__ __forceinline__ HeadRow hadamard_row(HeadRow x, int lane) {
   return bf16_row(make_float2(__fmul_rn(__fadd_rn(x.a.x, x.b.x), c), __fmul_rn(__fadd_rn(x.a.y, x.b.y), c)),
                   make_float2(__fmul_rn(__fsub_rn(x.a.x, x.b.x), c), __fmul_rn(__fsub_rn(x.a.y, x.b.y), c)));
 }
-// Eight E2M1 codes times their scale -> four words of bf16 pairs: at most 7 significant bits, exact.
+// The value of one E2M1 code.  Times its E4M3 scale it has at most 6 significant bits: exact in bf16.
 __device__ __forceinline__ float e2m1_value(uint32_t c) {
   const uint32_t mag = c & 7;
   const float mv = mag < 2 ? 0.5f * mag : __uint_as_float(((mag >> 1) + 126u) << 23 | (mag & 1u) << 22);
