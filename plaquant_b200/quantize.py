@@ -49,7 +49,7 @@ class QuantizedLinear:
         self.grouped, self.groupsize, self.clip_ratio = grouped, groupsize, clip_ratio
         self.online_had, self.had_matrix = online_had, had_matrix
         self.gemm_impl = "b200"
-        self._gemm_w = self._gemv_w = None
+        self._gemm_w = self._gemv_w = self._native = None
         if w_main_int.is_cuda:
             self._prepare()
 
@@ -133,7 +133,7 @@ class QuantizedLinear:
         if out is not None:
             rows = x.rows if isinstance(x, ops.PackedMatrix) else x.shape[:-1].numel()
             ops.check_out(out, rows, self.out_features, self._gemm_w.device)
-        if isinstance(x, torch.Tensor):
+        if isinstance(x, torch.Tensor) and type(self) is QuantizedLinear:      # a subclass may have its own quantize_input
             y = self.native().forward(x, self.online_had, norm_weight, eps, out)
             if y is not None:
                 return y

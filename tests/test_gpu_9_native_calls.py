@@ -150,6 +150,16 @@ def test_a_prompt_in_chunks_attends_like_the_whole_prompt(monkeypatch, head_dim,
     assert (got.float() - whole.float()).abs().max() <= 2.0 ** -8 * whole.float().abs().max()
     assert m.kv[0][0].shape[1] == 300
     ids = torch.randint(0, 100, (2, 40), generator=torch.Generator().manual_seed(6)).cuda()
+
+
+def test_a_subclass_quantises_its_own_way():
+    from plaquant_b200.quantize import QuantizedLinear
+
+    class Halved(QuantizedLinear):
+        def quantize_input(self, x, norm_weight=None, eps=1e-6):
+            return super().quantize_input(x * 0.5, norm_weight, eps)
+    w, x = synth_weight(256, 1024, seed=1).cuda(), synth_activation(5, 1024, seed=2).cuda()
+    assert torch.equal(Halved.from_weight(w)(x), QuantizedLinear.from_weight(w)(x * 0.5))
     m.forward(ids[:, :20])
     assert torch.isfinite(m.forward(ids[:, 20:], pos0=20, all_positions=True)).all()
     plq.check_device_status()
