@@ -343,7 +343,7 @@ PLQ_API int plq_gemv_static_scratch(const void* a_lo_codes, const void* a_lo_sf,
  * contract.  The weight rows are the 128-row side of the block-scaled tcgen05.mma and the m
  * activation rows the narrow side (N = 16 of the instruction), so the packed weights stream HBM -> shared memory -> tensor core
  * untouched by any thread.  When n gives fewer 128-row tiles than SMs, a thread-block cluster of up
- * to 8 CTAs shares each tile along K and combines the partial sums through distributed shared
+ * to 4 CTAs shares each tile along K and combines the partial sums through distributed shared
  * memory in a fixed order; no scratch memory is needed and results do not depend on timing.
  * The kernel is launched with programmatic stream serialisation: its set-up may run while the
  * previous kernel of the stream drains; it waits for that kernel's completion before it reads an
